@@ -71,6 +71,11 @@ void launch_body_constants(const Dev& d, const float4* lo, const float4* hi, con
 __global__ void k_integrate(Dev d, StepParams sp, float4* ox, float4* oq, float4* ov, float4* ow) {
     const float dt = sp.dt;
     const V3 g{sp.gx, sp.gy, sp.gz};
+    // The grid's counts and cursors of this tick (a memset each otherwise).
+    for (uint32_t i = grid_stride_begin(); i <= d.grid_size; i += grid_stride()) {
+        d.bucket_count[i] = 0u;
+        if (i < d.grid_size) d.bucket_cursor[i] = 0u;
+    }
     for (uint32_t i = grid_stride_begin(); i < d.n; i += grid_stride()) {
         const uint32_t motion = d.motion[i];
         float4 x = d.x[i], q = d.q[i], v = d.v[i], w = d.w[i];
@@ -227,7 +232,6 @@ void launch_pack_states(const Dev& d, uint32_t first, uint32_t count, float* dst
 }
 
 void launch_integrate(const Dev& d, const StepParams& sp, cudaStream_t s, const SolveBuffers& o) {
-    if (d.n_scenes > 1) cudaMemsetAsync(d.scene_hs, 0, sizeof(float) * d.n_scenes, s);
     k_integrate<<<blocks_for(d.n), kBlock, 0, s>>>(d, sp, o.ox, o.oq, o.ov, o.ow);
     note_launch(blocks_for(d.n));
     prof_mark(s, "integrate+proxy");
@@ -401,8 +405,8 @@ __global__ void k_query_count(Dev d) {
 }
 
 __global__ void k_query_write(Dev d) {
-    const uint32_t total = d.ctr->n_cand;
-    if (grid_stride_begin() == 0 && total > d.cap_cand) atomicOr(&d.ctr->status, kStCandidateOverflow);
+    // n_cand is the total clamped to the capacity (by the scan).
+    if (grid_stride_begin() == 0 && d.cand_off[d.n] > d.cap_cand) atomicOr(&d.ctr->status, kStCandidateOverflow);
     const uint32_t gl = threadIdx.x % kQueryLanes;
     const uint32_t gmask = ((1u << kQueryLanes) - 1u) << (threadIdx.x & 31u & ~(kQueryLanes - 1u));
     const uint32_t groups = grid_stride() / kQueryLanes;
@@ -433,25 +437,17 @@ __global__ void k_query_write(Dev d) {
     }
 }
 
-__global__ void k_clamp_count(uint32_t* count, uint32_t cap) {
-    if (*count > cap) *count = cap;
-}
-
 void launch_broadphase(const Dev& d, cudaStream_t s) {
     if (d.n_scenes > 1) {
-        cudaMemsetAsync(d.scene_large_count, 0, sizeof(uint32_t) * (d.n_scenes + 1), s);
-        cudaMemsetAsync(d.scene_large_cursor, 0, sizeof(uint32_t) * d.n_scenes, s);
         k_scene_large_count<<<blocks_for(d.n), kBlock, 0, s>>>(d);
         note_launch(blocks_for(d.n));
-        scan_u32(d.scene_large_count, d.scene_large_off, nullptr, d.n_scenes, nullptr, d.scan_tmp32, s);
+        scan_u32(d.scene_large_count, d.scene_large_off, nullptr, d.n_scenes, nullptr, 0u, d.scan_tmp32, s);
         k_scene_large_scatter<<<blocks_for(d.n), kBlock, 0, s>>>(d);
         note_launch(blocks_for(d.n));
     }
-    cudaMemsetAsync(d.bucket_count, 0, sizeof(uint32_t) * (d.grid_size + 1), s);
-    cudaMemsetAsync(d.bucket_cursor, 0, sizeof(uint32_t) * d.grid_size, s);
     k_grid_count<<<blocks_for(d.n), kBlock, 0, s>>>(d);
     note_launch(blocks_for(d.n));
-    scan_u32(d.bucket_count, d.bucket_off, nullptr, d.grid_size, nullptr, d.scan_tmp32, s);
+    scan_u32(d.bucket_count, d.bucket_off, nullptr, d.grid_size, nullptr, 0u, d.scan_tmp32, s);
     k_grid_scatter<<<blocks_for(d.n), kBlock, 0, s>>>(d);
     note_launch(blocks_for(d.n));
     prof_mark(s, "grid build");
@@ -463,11 +459,9 @@ void launch_broadphase(const Dev& d, cudaStream_t s) {
     k_query_count<<<blocks_for(kQueryLanes * d.n, 128), 128, 0, s>>>(d);
     note_launch(blocks_for(kQueryLanes * d.n, 128));
     prof_mark(s, "query count");
-    scan_u32(d.cand_count, d.cand_off, nullptr, d.n, &d.ctr->n_cand, d.scan_tmp32, s);
+    scan_u32(d.cand_count, d.cand_off, nullptr, d.n, &d.ctr->n_cand, d.cap_cand, d.scan_tmp32, s);
     k_query_write<<<blocks_for(kQueryLanes * d.n, 128), 128, 0, s>>>(d);
     note_launch(blocks_for(kQueryLanes * d.n, 128));
-    k_clamp_count<<<1, 1, 0, s>>>(&d.ctr->n_cand, d.cap_cand);
-    note_launch(1);
     prof_mark(s, "query write");
 }
 

@@ -246,7 +246,7 @@ extern "C" int pmb_mesh_bvh_build(const float* vertices, uint32_t vertex_count, 
                 uint32_t* kd = word == 0 ? kt[0] : (word == 1 ? ks[0] : kp[0]);
                 k_bvh_hist<<<tgrid, 64, 0, s>>>(kd, 8 * byte, n, tiles, hist);
                 note_launch(tgrid);
-                scan_u32(hist, offs, nullptr, 256 * tiles, nullptr, scan_tmp, s);
+                scan_u32(hist, offs, nullptr, 256 * tiles, nullptr, 0u, scan_tmp, s);
                 k_bvh_scatter<<<tgrid, 64, 0, s>>>(kd, 8 * byte, n, tiles, offs, kp[0], ks[0], kt[0], val[0], kp[1],
                                                    ks[1], kt[1], val[1]);
                 note_launch(tgrid);

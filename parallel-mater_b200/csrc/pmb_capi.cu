@@ -156,13 +156,21 @@ StepParams params_from(const pmb_step_desc& s) {
     return p;
 }
 
-__global__ void k_reset_counters(Counters* c) {
+// Also the per-scene sums that the predictor and the large-body lists add to.
+__global__ void k_reset_counters(Dev d) {
     // bar_gen is left alone: it only ever increases.
-    uint32_t* w = reinterpret_cast<uint32_t*>(c);
+    uint32_t* w = reinterpret_cast<uint32_t*>(d.ctr);
     const uint32_t words = sizeof(Counters) / 4;
     const uint32_t skip = offsetof(Counters, bar_gen) / 4;
     for (uint32_t i = threadIdx.x; i < words; i += blockDim.x)
         if (i != skip) w[i] = 0;
+    if (d.n_scenes > 1)
+        for (uint32_t i = threadIdx.x; i <= d.n_scenes; i += blockDim.x) {
+            d.scene_large_count[i] = 0;
+            if (i == d.n_scenes) break;
+            d.scene_large_cursor[i] = 0;
+            d.scene_hs[i] = 0.0f;
+        }
 }
 
 void enqueue_step(pmb_world* w, const StepParams& sp) {
@@ -171,7 +179,7 @@ void enqueue_step(pmb_world* w, const StepParams& sp) {
     w->ledger = LaunchLedger{};
     g_ledger = &w->ledger;
     set_phase(kPhBoundary);
-    k_reset_counters<<<1, 256, 0, s>>>(d.ctr);
+    k_reset_counters<<<1, 1024, 0, s>>>(d);
     note_launch(1);
     set_phase(kPhPredict);
     launch_integrate(d, sp, s, w->out);

@@ -42,6 +42,7 @@ __global__ void k_prepare_bodies(Dev d, StepParams sp) {
         d.jdeg[i] = 0;
         d.inc_cursor[i] = 0;
         d.jinc_cursor[i] = 0;
+        d.cdirty[i] = d.cdirty[size_t(d.n) + i] = 0;
         if (d.motion[i] != kDynamic) {
             d.color[i] = kInvalid;
             d.prev_vel[i] = make_float4(0, 0, 0, 0);
@@ -546,15 +547,15 @@ void launch_graph(const Dev& d, const StepParams& sp, cudaStream_t s, int coop_b
     uint32_t gb = cap_blocks(d.cap_pair > d.nj ? d.cap_pair : d.nj);
     k_graph_degrees<<<gb, kBlock, 0, s>>>(d, sp);
     note_launch(gb);
-    scan_u32(d.deg, d.inc_off, nullptr, d.n, nullptr, d.scan_tmp32, s);
-    scan_u32(d.jdeg, d.jinc_off, nullptr, d.n, nullptr, d.scan_tmp32, s);
+    scan_u32(d.deg, d.inc_off, nullptr, d.n, nullptr, 0u, d.scan_tmp32, s);
+    scan_u32(d.jdeg, d.jinc_off, nullptr, d.n, nullptr, 0u, d.scan_tmp32, s);
     k_graph_fill<<<gb, kBlock, 0, s>>>(d);
     note_launch(gb);
     k_graph_lists<<<blocks_for(d.n), kBlock, 0, s>>>(d);
     note_launch(blocks_for(d.n));
     k_graph_roots<<<blocks_for(d.n), kBlock, 0, s>>>(d);
     note_launch(blocks_for(d.n));
-    scan_u32(d.rcount, d.roff, nullptr, d.n, nullptr, d.scan_tmp32, s);
+    scan_u32(d.rcount, d.roff, nullptr, d.n, nullptr, 0u, d.scan_tmp32, s);
     k_row_lists<<<blocks_for(d.n), kBlock, 0, s>>>(d);
     note_launch(blocks_for(d.n));
     k_graph_impact<<<cap_blocks(d.cap_pair), kBlock, 0, s>>>(d);
@@ -564,7 +565,6 @@ void launch_graph(const Dev& d, const StepParams& sp, cudaStream_t s, int coop_b
     prof_mark(s, "graph lists+islands");
     k_neighbour_lists<<<blocks_for(d.n), kBlock, 0, s>>>(d);
     note_launch(blocks_for(d.n));
-    cudaMemsetAsync(d.cdirty, 0, 2 * size_t(d.n), s);
     void* args[] = {const_cast<Dev*>(&d)};
     cudaLaunchCooperativeKernel(color_kernel_ptr, dim3(coop_blocks), dim3(kColorThreads), args, 0, s);
     note_launch(coop_blocks);

@@ -1,8 +1,13 @@
 // SPDX-License-Identifier: MIT
 // Device-wide exclusive prefix sums whose length is read from device memory,
 // so compaction stages (candidate pairs, contacts) need no host round trip.
-// Three passes: per-tile totals, one-block scan of the tile totals, per-tile
-// scan with the tile's offset. Tiles are 2048 elements (256 threads x 8).
+//
+// A tick makes nine of them, most over a few thousand elements, where the
+// launches are the cost (about 2 us each, against 0.1 us of memory time for
+// 32,768 words). So a scan whose capacity fits one block's few rounds is one
+// launch (k_scan_block); a longer one is two: per-tile totals, then every
+// tile's block adds up the totals before its own (at most a few thousand
+// words, read by 256 threads at once) instead of waiting for a pass over them.
 #include "pmb_world.cuh"
 
 namespace pmb {
@@ -10,9 +15,12 @@ namespace pmb {
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 8;
 constexpr uint32_t kScanTile = kScanThreads * kScanItems;
+constexpr int kScanBlockThreads = 1024;
+// Longest capacity scanned by one block: four rounds of 8,192 elements.
+constexpr uint32_t kScanBlockMost = 4u * kScanBlockThreads * kScanItems;
 
-template <class T> __device__ T block_exclusive_scan(T v, T* total) {
-    __shared__ T warp_sums[kScanThreads / 32];
+template <class T, int kThreads> __device__ T block_exclusive_scan(T v, T* total) {
+    __shared__ T warp_sums[kThreads / 32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     T inc = v;
 #pragma unroll
@@ -23,15 +31,15 @@ template <class T> __device__ T block_exclusive_scan(T v, T* total) {
     if (lane == 31) warp_sums[wid] = inc;
     __syncthreads();
     if (wid == 0) {
-        T s = lane < kScanThreads / 32 ? warp_sums[lane] : T(0);
+        T s = lane < kThreads / 32 ? warp_sums[lane] : T(0);
         T si = s;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             T y = __shfl_up_sync(0xffffffffu, si, o);
             if (lane >= o) si += y;
         }
-        if (lane < kScanThreads / 32) warp_sums[lane] = si - s;
-        if (lane == kScanThreads / 32 - 1 && total) *total = si;
+        if (lane < kThreads / 32) warp_sums[lane] = si - s;
+        if (lane == kThreads / 32 - 1 && total) *total = si;
     }
     __syncthreads();
     T r = inc - v + warp_sums[wid];
@@ -39,102 +47,105 @@ template <class T> __device__ T block_exclusive_scan(T v, T* total) {
     return r;
 }
 
-template <class T>
-__global__ void k_tile_sums(const T* in, const uint32_t* count_ptr, uint32_t capacity, T* tile_sums) {
-    uint32_t count = count_ptr ? min(*count_ptr, capacity) : capacity;
-    uint32_t base = blockIdx.x * kScanTile;
-    T s = 0;
-    if (base < count) {
-        for (int k = 0; k < kScanItems; ++k) {
-            uint32_t i = base + threadIdx.x * kScanItems + k;
-            if (i < count) s += in[i];
-        }
-    }
-    __shared__ T total;
-    block_exclusive_scan<T>(s, &total);
-    if (threadIdx.x == 0) tile_sums[blockIdx.x] = total;
-}
-
-template <class T> __global__ void k_scan_tiles(T* tile_sums, uint32_t tiles, T* grand_total) {
-    // One block: each thread owns a contiguous run of tile sums.
-    const uint32_t per = (tiles + kScanThreads - 1) / kScanThreads;
-    uint32_t b = threadIdx.x * per;
-    T s = 0;
-    for (uint32_t k = 0; k < per; ++k)
-        if (b + k < tiles) s += tile_sums[b + k];
-    __shared__ T total;
-    T off = block_exclusive_scan<T>(s, &total);
-    for (uint32_t k = 0; k < per; ++k) {
-        if (b + k < tiles) {
-            T v = tile_sums[b + k];
-            tile_sums[b + k] = off;
-            off += v;
-        }
-    }
-    if (threadIdx.x == 0 && grand_total) *grand_total = total;
-}
-
-template <class T>
-__global__ void k_scan_apply(const T* in, T* out, const uint32_t* count_ptr, uint32_t capacity, const T* tile_sums) {
-    uint32_t count = count_ptr ? min(*count_ptr, capacity) : capacity;
-    uint32_t base = blockIdx.x * kScanTile;
-    if (base >= count) return;
-    T vals[kScanItems];
+// This thread's kScanItems elements from `first` on (zeros past `count`).
+template <class T> __device__ __forceinline__ T load_items(const T* in, uint32_t first, uint32_t count, T* vals) {
     T s = 0;
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) {
-        uint32_t i = base + threadIdx.x * kScanItems + k;
-        vals[k] = i < count ? in[i] : T(0);
+        vals[k] = first + k < count ? in[first + k] : T(0);
         s += vals[k];
     }
-    T off = block_exclusive_scan<T>(s, nullptr) + tile_sums[blockIdx.x];
+    return s;
+}
+template <class T>
+__device__ __forceinline__ void store_items(T* out, uint32_t first, uint32_t count, const T* vals, T off) {
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) {
-        uint32_t i = base + threadIdx.x * kScanItems + k;
-        if (i < count) out[i] = off;
+        if (first + k < count) out[first + k] = off;
         off += vals[k];
     }
 }
 
 template <class T>
-__global__ void k_scan_total(T* out, const uint32_t* count_ptr, uint32_t capacity, const T* grand_total) {
-    uint32_t count = count_ptr ? min(*count_ptr, capacity) : capacity;
-    out[count] = *grand_total;
+__global__ void __launch_bounds__(kScanBlockThreads)
+    k_scan_block(const T* in, T* out, const uint32_t* count_ptr, uint32_t capacity, T* total, uint32_t total_cap) {
+    const uint32_t count = count_ptr ? min(*count_ptr, capacity) : capacity;
+    __shared__ T chunk;
+    T carry = 0;
+    for (uint32_t base = 0; base < count; base += kScanBlockThreads * kScanItems) {
+        const uint32_t first = base + threadIdx.x * kScanItems;
+        T vals[kScanItems];
+        const T s = load_items(in, first, count, vals);
+        const T off = block_exclusive_scan<T, kScanBlockThreads>(s, &chunk) + carry;
+        store_items(out, first, count, vals, off);
+        carry += chunk;
+    }
+    if (threadIdx.x == 0) {
+        out[count] = carry;
+        if (total) *total = carry < T(total_cap) ? carry : T(total_cap);
+    }
 }
 
 template <class T>
-static void scan_impl(const T* in, T* out, const uint32_t* count_ptr, uint32_t capacity, T* tmp, cudaStream_t s) {
-    uint32_t tiles = (capacity + kScanTile - 1) / kScanTile;
-    if (tiles == 0) tiles = 1;
-    k_tile_sums<T><<<tiles, kScanThreads, 0, s>>>(in, count_ptr, capacity, tmp);
-    note_launch(tiles);
-    k_scan_tiles<T><<<1, kScanThreads, 0, s>>>(tmp, tiles, tmp + tiles);
-    note_launch(1);
-    k_scan_apply<T><<<tiles, kScanThreads, 0, s>>>(in, out, count_ptr, capacity, tmp);
-    note_launch(tiles);
-    k_scan_total<T><<<1, 1, 0, s>>>(out, count_ptr, capacity, tmp + tiles);
-    note_launch(1);
+__global__ void k_tile_sums(const T* in, const uint32_t* count_ptr, uint32_t capacity, T* tile_sums) {
+    const uint32_t count = count_ptr ? min(*count_ptr, capacity) : capacity;
+    const uint32_t base = blockIdx.x * kScanTile;
+    if (base >= count) return;  // totals past the end are never read
+    T vals[kScanItems];
+    const T s = load_items(in, base + threadIdx.x * kScanItems, count, vals);
+    __shared__ T total;
+    block_exclusive_scan<T, kScanThreads>(s, &total);
+    if (threadIdx.x == 0) tile_sums[blockIdx.x] = total;
 }
 
-// out must hold capacity + 1 entries; out[count] receives the total and, when
-// total is non-null, so does *total.
-__global__ void k_copy_total(const uint32_t* out, const uint32_t* count_ptr, uint32_t capacity, uint32_t* total) {
-    uint32_t count = count_ptr ? min(*count_ptr, capacity) : capacity;
-    *total = out[count];
+template <class T>
+__global__ void k_scan_apply(const T* in, T* out, const uint32_t* count_ptr, uint32_t capacity, const T* tile_sums,
+                             T* total, uint32_t total_cap) {
+    const uint32_t count = count_ptr ? min(*count_ptr, capacity) : capacity;
+    const uint32_t base = blockIdx.x * kScanTile;
+    if (base >= count && !(blockIdx.x == 0 && count == 0)) return;
+    T before = 0;
+    for (uint32_t k = threadIdx.x; k < blockIdx.x; k += kScanThreads) before += tile_sums[k];
+    __shared__ T start, tile;
+    block_exclusive_scan<T, kScanThreads>(before, &start);
+    const T carry = start;
+    const uint32_t first = base + threadIdx.x * kScanItems;
+    T vals[kScanItems];
+    const T s = load_items(in, first, count, vals);
+    const T off = block_exclusive_scan<T, kScanThreads>(s, &tile) + carry;
+    store_items(out, first, count, vals, off);
+    if (threadIdx.x == 0 && count - base <= kScanTile) {  // the last tile
+        const T all = carry + tile;
+        out[count] = all;
+        if (total) *total = all < T(total_cap) ? all : T(total_cap);
+    }
+}
+
+// out holds capacity + 1 entries; out[count] receives the total and, when
+// `total` is non-null, *total the total or `total_cap` if that is less.
+template <class T>
+static void scan_impl(const T* in, T* out, const uint32_t* count_ptr, uint32_t capacity, T* total, uint32_t total_cap,
+                      T* tmp, cudaStream_t s) {
+    if (capacity <= kScanBlockMost) {
+        k_scan_block<T><<<1, kScanBlockThreads, 0, s>>>(in, out, count_ptr, capacity, total, total_cap);
+        note_launch(1);
+        return;
+    }
+    const uint32_t tiles = (capacity + kScanTile - 1) / kScanTile;
+    k_tile_sums<T><<<tiles, kScanThreads, 0, s>>>(in, count_ptr, capacity, tmp);
+    note_launch(tiles);
+    k_scan_apply<T><<<tiles, kScanThreads, 0, s>>>(in, out, count_ptr, capacity, tmp, total, total_cap);
+    note_launch(tiles);
 }
 
 void scan_u32(const uint32_t* in, uint32_t* out, const uint32_t* count_ptr, uint32_t capacity, uint32_t* total,
-              uint32_t* tmp, cudaStream_t s) {
-    scan_impl<uint32_t>(in, out, count_ptr, capacity, tmp, s);
-    if (total) {
-        k_copy_total<<<1, 1, 0, s>>>(out, count_ptr, capacity, total);
-        note_launch(1);
-    }
+              uint32_t total_cap, uint32_t* tmp, cudaStream_t s) {
+    scan_impl<uint32_t>(in, out, count_ptr, capacity, total, total_cap, tmp, s);
 }
 
 void scan_u64(const uint64_t* in, uint64_t* out, const uint32_t* count_ptr, uint32_t capacity, uint64_t* tmp,
               cudaStream_t s) {
-    scan_impl<uint64_t>(in, out, count_ptr, capacity, tmp, s);
+    scan_impl<uint64_t>(in, out, count_ptr, capacity, nullptr, 0u, tmp, s);
 }
 
 }  // namespace pmb

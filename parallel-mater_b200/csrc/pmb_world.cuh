@@ -356,7 +356,7 @@ void launch_solve_all(const Dev& d, const StepParams& sp, cudaStream_t s, const 
 void launch_body_constants(const Dev& d, const float4* lo, const float4* hi, const float4* sph, cudaStream_t s);
 void launch_finish(const Dev& d, const StepParams& sp, cudaStream_t s);
 void scan_u32(const uint32_t* in, uint32_t* out, const uint32_t* count_ptr, uint32_t capacity, uint32_t* total,
-              uint32_t* tmp, cudaStream_t s);
+              uint32_t total_cap, uint32_t* tmp, cudaStream_t s);
 void scan_u64(const uint64_t* in, uint64_t* out, const uint32_t* count_ptr, uint32_t capacity, uint64_t* tmp,
               cudaStream_t s);
 int coop_blocks_for(const void* kernel, int threads, size_t smem);
