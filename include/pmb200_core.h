@@ -201,8 +201,10 @@ PMB_API int pmb_world_solve_timer(pmb_world* world, int enable, float* total_ms,
  * memory; `node_count` (host) receives the node count, and a capacity below
  * it returns PMB_ERROR_CAPACITY_EXCEEDED; an index at or past `vertex_count`
  * returns PMB_ERROR_INVALID_ARGUMENT before any other device work. Work runs on `stream` (CUDA
- * stream, null for the default); the call allocates scratch with cudaMalloc
- * and returns after the stream has finished. */
+ * stream, null for the default); the call takes scratch (104 bytes a triangle
+ * and some) from a pool of the current device that keeps at most 64 MiB
+ * between calls, emptied when a world of that device is destroyed, and
+ * returns after the stream has finished. */
 PMB_API int pmb_mesh_bvh_build(const float* vertices, uint32_t vertex_count, const uint32_t* indices,
                                uint32_t index_count, uint32_t* order, float* nodes, uint32_t node_capacity,
                                uint32_t* node_count, void* stream);

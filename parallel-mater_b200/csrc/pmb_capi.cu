@@ -745,6 +745,7 @@ void pmb_world_destroy(pmb_world* w) {
     for (void* p : w->snapshot) cudaFree(p);
     for (void* p : w->mlp.allocs) cudaFree(p);
     if (w->own_stream && w->stream) cudaStreamDestroy(w->stream);
+    release_bvh_scratch(w->device);
     delete w;
 }
 

@@ -359,6 +359,7 @@ void scan_u32(const uint32_t* in, uint32_t* out, const uint32_t* count_ptr, uint
               uint32_t total_cap, uint32_t* tmp, cudaStream_t s);
 void scan_u64(const uint64_t* in, uint64_t* out, const uint32_t* count_ptr, uint32_t capacity, uint64_t* tmp,
               cudaStream_t s);
+void release_bvh_scratch(int device);  // gives back the mesh BVH builds' kept scratch
 int coop_blocks_for(const void* kernel, int threads, size_t smem);
 // Stage timing for diagnosis: records a CUDA event named `stage` when a
 // profiled step is being enqueued (never during graph capture).

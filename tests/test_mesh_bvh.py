@@ -108,6 +108,15 @@ def test_device_builder_equals_the_host_tree(gpu_available, name, vertices, indi
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("triangles", [2, 8, 9, 511, 512, 513, 1023, 1025, 2047, 2049, 4097, 11111])
+def test_device_builder_at_the_edges_of_its_tiles(gpu_available, triangles):
+    """Subtrees of at most 512 triangles are built by one block, larger nodes
+    level by level over 2,048-key radix tiles: sizes around those edges, on a
+    coarse grid (many equal centroids), against the restated builder."""
+    test_device_builder_equals_the_host_tree(True, "soup", *_grid_soup(triangles, triangles, cells=9))
+
+
+@pytest.mark.gpu
 def test_device_builder_rejects_out_of_range_indices(gpu_available):
     import torch
     dev = torch.device("cuda", 0)
