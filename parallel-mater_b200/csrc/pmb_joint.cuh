@@ -308,4 +308,216 @@ static __device__ float visit_joint(const Joint& o, JointRow* rows, const BodyVi
     return c.impulse;
 }
 
+// ---- joint rows by lanes
+//
+// A sweep visits every joint three times (its two bodies' colours, the dual
+// pass), and a visit re-linearises up to 18 rows. In one thread that is a
+// chain of 20-30 us a body; the three axes of a joint are independent, so a
+// lane takes one axis (and a group several joints at once), and what depends
+// only on the tick's start -- the joint's errors at the previous poses, which
+// rows it has -- is formed once by the preparation (JointOld, JointState::rows).
+struct JointOld {
+    V3 lin, rot, twist;  // the rows' values at the previous poses, per axis
+    Q4 rel;              // motors: the relative frame
+};
+constexpr uint32_t kOldWords = 4;  // float4 per joint
+
+// Row kinds of an axis half (linear, angular), in the order they are visited;
+// kLimit: the equality, or the upper bound.
+enum : unsigned { kRowLock = 0, kRowLimit = 1, kRowLower = 2, kRowSpring = 3, kRowMotor = 4, kRowKinds = 5 };
+constexpr unsigned kAxisBits = 2 * kRowKinds;
+constexpr uint32_t kAxisMask = (1u << kAxisBits) - 1u;
+
+__device__ __forceinline__ bool joint_swings(const Joint& o) {
+    return o.type == kHinge || o.type == kPiston || (o.type == kMotor && o.motor_angular != 0);
+}
+__device__ __forceinline__ V3 joint_free_axis(uint32_t type) {
+    return type == kHinge ? V3{0, 0, 1} : V3{1, 0, 0};
+}
+
+// The rows of joint o (bit axis * kAxisBits + angular * kRowKinds + kind),
+// by the conditions of geometry_constraints.slang:780-920.
+__device__ __forceinline__ uint32_t joint_row_mask(const Joint& o) {
+    const uint32_t t = o.type;
+    const bool generic = t == kGeneric || t == kGenericSpring, motor = t == kMotor;
+    uint32_t mask = 0;
+    for (unsigned axis = 0; axis < 3; ++axis)
+        for (unsigned av = 0; av < (t == kPoint ? 1u : 2u); ++av) {
+            const bool angular = av != 0;
+            uint32_t m = 0;
+            const bool lock = angular ? (t == kFixed || t == kSlider || (t == kHinge && axis != 2) ||
+                                         (t == kPiston && axis != 0) || (motor && (axis != 0 || o.motor_angular == 0)))
+                                      : (t == kFixed || t == kPoint || t == kHinge ||
+                                         ((t == kSlider || t == kPiston) && axis != 0) ||
+                                         (motor && (axis != 0 || o.motor_linear == 0)));
+            if (lock) m |= 1u << kRowLock;
+            const bool free_limit = angular ? ((t == kHinge && axis == 2) || (t == kPiston && axis == 0))
+                                            : ((t == kSlider || t == kPiston) && axis == 0);
+            if ((generic || free_limit) && ((angular ? o.ang_limit_axes : o.lin_limit_axes) & (1u << axis)) != 0) {
+                const float lower = angular ? o.ang_lower[axis] : o.lin_lower[axis];
+                const float upper = angular ? o.ang_upper[axis] : o.lin_upper[axis];
+                if (lower == upper) m |= 1u << kRowLimit;
+                else if (lower < upper) m |= (1u << kRowLimit) | (1u << kRowLower);
+            }
+            if (t == kGenericSpring && ((angular ? o.ang_spring_axes : o.lin_spring_axes) & (1u << axis)) != 0)
+                m |= 1u << kRowSpring;
+            if (motor && axis == 0 && (angular ? o.motor_angular != 0 : o.motor_linear != 0)) m |= 1u << kRowMotor;
+            mask |= m << (axis * kAxisBits + av * kRowKinds);
+        }
+    return mask;
+}
+
+// The joint's geometry at one pair of poses.
+struct JointPose {
+    V3 arm_a, arm_b, error;
+    Q4 frame_a, frame_b;
+    V3 twist, swing_axis, rotation;
+};
+__device__ __forceinline__ JointPose joint_pose(const Joint& o, V3 xa, Q4 qa, V3 xb, Q4 qb) {
+    JointPose p;
+    p.arm_a = rotate(qa, V3{o.anchor_a[0], o.anchor_a[1], o.anchor_a[2]});
+    p.arm_b = rotate(qb, V3{o.anchor_b[0], o.anchor_b[1], o.anchor_b[2]});
+    p.error = sub(add(xb, p.arm_b), add(xa, p.arm_a));
+    p.frame_a = qnormalize(qmul(qa, Q4{o.frame_a[0], o.frame_a[1], o.frame_a[2], o.frame_a[3]}));
+    p.frame_b = Q4{0, 0, 0, 1};
+    p.twist = p.swing_axis = p.rotation = V3{0, 0, 0};
+    if (o.type != kPoint) {
+        p.frame_b = qnormalize(qmul(qb, Q4{o.frame_b[0], o.frame_b[1], o.frame_b[2], o.frame_b[3]}));
+        p.twist = rotation_vector(qrelative(p.frame_a, p.frame_b, true));
+        const V3 free_axis = joint_free_axis(o.type);
+        p.swing_axis = inv_rotate(p.frame_a, rotate(p.frame_b, free_axis));
+        p.rotation = joint_swings(o) ? cross(free_axis, p.swing_axis) : p.twist;
+    }
+    return p;
+}
+__device__ __forceinline__ void store_joint_old(const Joint& o, V3 xa, Q4 qa, V3 xb, Q4 qb, float4* out) {
+    const JointPose p = joint_pose(o, xa, qa, xb, qb);
+    float lin[3];
+    for (unsigned axis = 0; axis < 3; ++axis) lin[axis] = dot(p.error, rotate(p.frame_a, unit_axis(axis)));
+    const Q4 rel = o.type == kMotor ? qrelative(p.frame_a, p.frame_b, true) : Q4{0, 0, 0, 1};
+    out[0] = make_float4(lin[0], lin[1], lin[2], p.rotation.x);
+    out[1] = make_float4(p.rotation.y, p.rotation.z, p.twist.x, p.twist.y);
+    out[2] = make_float4(p.twist.z, rel.x, rel.y, rel.z);
+    out[3] = make_float4(rel.w, 0.0f, 0.0f, 0.0f);
+}
+__device__ __forceinline__ JointOld load_joint_old(const float4* r, uint32_t type) {
+    JointOld o;
+    const float4 a = r[0];
+    o.lin = V3{a.x, a.y, a.z};
+    o.rot = o.twist = V3{0, 0, 0};
+    o.rel = Q4{0, 0, 0, 1};
+    if (type != kPoint) {
+        const float4 b = r[1], c = r[2];
+        o.rot = V3{a.w, b.x, b.y};
+        o.twist = V3{b.z, b.w, c.x};
+        if (type == kMotor) o.rel = Q4{c.y, c.z, c.w, r[3].x};
+    }
+    return o;
+}
+
+// One row at the current poses: its jacobians, error and force, as joint_row
+// forms them (geometry_constraints.slang:626-713) from the stored dual.
+struct LaneRow {
+    V6 ja, jb;
+    float force, stiff;              // force within the bounds; stiffness of the block's term
+    float error;                     // C at the current displacements (row_error)
+    float lower, upper, stiffness;   // kMaxPenalty: a hard row
+};
+__device__ __forceinline__ LaneRow lane_row(const Joint& o, const JointPose& p, const JointOld& old, V3 dir,
+                                            unsigned axis, bool angular, unsigned kind, const V6& dxa, const V6& dxb,
+                                            Dual dual, float dt) {
+    LaneRow r;
+    float current, previous, stab = kAlpha, damping = 0.0f, stiffness = kMaxPenalty, speed = 0.0f;
+    r.lower = -kMaxPenalty;
+    r.upper = kMaxPenalty;
+    const bool limit = kind == kRowLimit || kind == kRowLower, motor = kind == kRowMotor;
+    V3 mrot{0, 0, 0};
+    if (angular) {
+        V3 ax;
+        if (motor) {
+            const Q4 rel = qrelative(p.frame_a, p.frame_b, true);
+            mrot = rotation_vector(qrelative(Q4{0, 0, 0, 1}, qrelative(old.rel, rel, false), true));
+        }
+        if (joint_swings(o) && !limit && !motor) {
+            const V3 free_axis = joint_free_axis(o.type);
+            ax = rotate(p.frame_a, sub(mul(unit_axis(axis), dot(free_axis, p.swing_axis)),
+                                       mul(free_axis, comp(p.swing_axis, axis))));
+        } else {
+            ax = log_axis(p.frame_a, motor ? mrot : p.twist, axis);
+        }
+        r.ja = jac(V3{0, 0, 0}, mul(ax, -1.0f));
+        r.jb = jac(V3{0, 0, 0}, ax);
+        current = comp(limit ? p.twist : p.rotation, axis);
+        previous = comp(limit ? old.twist : old.rot, axis);
+    } else {
+        r.ja = jac(mul(dir, -1.0f), add(mul(cross(p.arm_a, dir), -1.0f), cross(dir, p.error)));
+        r.jb = jac(dir, cross(p.arm_b, dir));
+        current = dot(p.error, dir);
+        previous = comp(old.lin, axis);
+    }
+    if (limit) {
+        const float lower = angular ? o.ang_lower[axis] : o.lin_lower[axis];
+        const float upper = angular ? o.ang_upper[axis] : o.lin_upper[axis];
+        if (kind == kRowLower) {
+            current = current - lower;
+            previous = fmn(previous - lower, 0.0f);
+            r.upper = 0.0f;
+            stab = 0.8f;
+        } else if (lower == upper) {
+            current = current - lower;
+            previous = previous - lower;
+        } else {
+            current = current - upper;
+            previous = fmx(previous - upper, 0.0f);
+            r.lower = 0.0f;
+            stab = 0.8f;
+        }
+    } else if (kind == kRowSpring) {
+        stiffness = angular ? o.ang_stiffness[axis] : o.lin_stiffness[axis];
+        damping = angular ? o.ang_damping[axis] : o.lin_damping[axis];
+    } else if (motor) {
+        speed = angular ? o.motor_angular_velocity : o.motor_linear_velocity;
+        const float bound = (angular ? o.motor_angular_max_impulse : o.motor_linear_max_impulse) / dt;
+        r.lower = -bound;
+        r.upper = bound;
+        current = (angular ? comp(mrot, axis) : current - previous) - speed * dt;
+        previous = 0.0f;
+    }
+    r.stiffness = stiffness;
+    const float moved_a = dot6(r.ja, dxa), moved_b = dot6(r.jb, dxb);
+    const float disp = moved_a + moved_b;
+    const float error = current - (stiffness < kMaxPenalty ? 0.0f : stab * previous) - disp;
+    r.error = error + moved_a + moved_b;
+    // trial = base + damping (velocity + disp / dt): without damping that
+    // term is a zero, which changes nothing unless base is one too (or the
+    // velocity is not finite), so its two divisions are left out.
+    const float base = dual.lambda + dual.penalty * (error + disp);
+    const float moved = current - previous - disp;
+    float trial = base;
+    r.stiff = dual.penalty;
+    if (damping != 0.0f || base == 0.0f || !(fab(moved) < 1.0e37f * dt) || !(fab(disp) < 1.0e37f * dt) ||
+        (motor && !(fab(speed) < 1.0e37f))) {
+        const float velocity = motor ? speed : moved / dt;
+        trial = dual.lambda + dual.penalty * (error + disp) + damping * (velocity + disp / dt);
+        r.stiff = dual.penalty + damping / dt;
+    }
+    r.force = fclamp(trial, r.lower, r.upper);
+    const bool two_sided = r.lower < 0.0f && r.upper > 0.0f;
+    if (!(two_sided || (trial > r.lower && trial < r.upper))) r.stiff = 0.0f;
+    return r;
+}
+
+// The linear rows' curvature terms of the block's angular diagonal
+// (geometry_constraints.slang:668-684), for the body with arm `arm`.
+__device__ __forceinline__ V3 lane_curvature(V3 axis, V3 arm, float force) {
+    float out[3];
+#pragma unroll
+    for (unsigned col = 0; col < 3; ++col) {
+        const V3 val = sub(mul(add(mul(axis, comp(arm, col)), mul(arm, comp(axis, col))), 0.5f),
+                           mul(unit_axis(col), dot(axis, arm)));
+        out[col] = fab(force) * sqrtf(len2(val));
+    }
+    return {out[0], out[1], out[2]};
+}
+
 }  // namespace pmb

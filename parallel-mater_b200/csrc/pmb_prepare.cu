@@ -189,6 +189,8 @@ __global__ void k_prepare_joints(Dev d, StepParams sp) {
                 visit_joint(o, d.jrows + size_t(j) * 18, A, B, v3(d.x[a]), q4(d.q[a]), v3(d.x[b]), q4(d.q[b]),
                             d.p0[a], d.p0[b], dt, &scratch, true, kVisitInit, &count);
                 st.count = count;
+                st.rows = joint_row_mask(o);
+                store_joint_old(o, v3(d.x[a]), q4(d.q[a]), v3(d.x[b]), q4(d.q[b]), d.jold + size_t(j) * kOldWords);
             }
         }
         d.jstate[j] = st;

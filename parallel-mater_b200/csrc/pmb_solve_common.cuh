@@ -117,8 +117,6 @@ template <int G> struct GroupRowsData {
     // per entry.
     float r[G][kSlotWords];
     float nrow[kSlots][9];  // normal row: jacobian[6], raw penalty, trial force (and a pad word)
-    Blk jblk;            // the block while joint rows are added (joint_rows_shared)
-    BodyView jview[2];   // the joint's two bodies during its visit
 };
 template <int G> struct GroupRows : GroupRowsData<G> {
     // Pads the group to 24 banks mod 32 (8 lanes: bases 0, 24, 16, 8) or 16
@@ -135,13 +133,11 @@ static_assert(sizeof(GroupRows<8>) / 4 % 32 == 24 && sizeof(GroupRows<16>) / 4 %
 // 32-lane group.
 constexpr size_t kWarpStage = 4 * sizeof(GroupRows<8>);
 static_assert(2 * sizeof(GroupRows<16>) <= kWarpStage && sizeof(GroupRows<32>) <= kWarpStage, "staging area");
-// Per-thread slots of the body-per-thread sweep and the dual pass: a block,
-// a joint's two body views and its residual contributions, in shared memory
-// so the joint visit (a call) reads them there rather than from local memory.
+// Per-thread slots of the body-per-thread sweep: a block and a joint's two
+// body views, in shared memory so the joint visit (a call) reads them there
+// rather than from local memory.
 constexpr size_t kThreadViews = 32 * sizeof(Blk);
-constexpr size_t kThreadJointRes = kThreadViews + 64 * sizeof(BodyView);
-static_assert(kThreadViews % 8 == 0 && kThreadJointRes % 8 == 0, "slot alignment");
-static_assert(kThreadJointRes + 32 * sizeof(JointRes) <= kWarpStage, "per-thread joint slots");
+static_assert(kThreadViews + 64 * sizeof(BodyView) <= kWarpStage, "per-thread joint slots");
 
 __device__ __forceinline__ void entry_ik(int e, int& i, int& k) {
     i = e >= 15 ? 5 : e >= 10 ? 4 : e >= 6 ? 3 : e >= 3 ? 2 : e >= 1 ? 1 : 0;
@@ -400,6 +396,146 @@ __device__ __forceinline__ void joint_rows_shared(const Dev& d, uint32_t i, uint
     __syncwarp(gmask);
 }
 
+// The two bodies of a joint as its rows read them during a sweep.
+struct JointEnds {
+    V6 dxa, dxb;
+    V3 xa, xb;
+    Q4 qa, qb;
+};
+__device__ __forceinline__ void load_end(const Dev& d, uint32_t i, V6& dx, V3& x, Q4& q) {
+    const float4 tx = d.tx[i], tq = d.tq[i], l = d.dxl[i], a = d.dxa[i], dq = d.dq[i];
+    dx = {{l.x, l.y, l.z, a.x, a.y, a.z}};
+    x = add(v3(tx), v3(l));
+    q = q4(tq);
+    if (dq.x != 0.0f || dq.y != 0.0f || dq.z != 0.0f) q = qnormalize(qmul(q4(dq), q));  // body_pose
+}
+__device__ __forceinline__ JointEnds load_ends(const Dev& d, uint32_t a, uint32_t b) {
+    JointEnds e;
+    load_end(d, a, e.dxa, e.xa, e.qa);
+    load_end(d, b, e.dxb, e.xb, e.qb);
+    return e;
+}
+
+// Joint rows of body i added to its block entries by the group's lanes, in
+// the serial loop's order (joints in list order, then axes, then rows).
+// A lane takes one axis of one joint -- two, five or ten joints at a time
+// for 8, 16 and 32 lanes -- and stages its rows over the contact rows, which
+// are in the entries by now: a lane's 43 words hold three rows, the most an
+// axis of any joint but a generic or spring one has; a joint with more is
+// taken alone, its lanes' rows spread over the group's slots.
+constexpr int kJointWords = 12;  // jacobian[6], stiffness, force, curvature[3], whether it has one
+constexpr int kJointRowsMost = 6;
+template <int G>
+__device__ __forceinline__ void joint_rows_lanes(const Dev& d, uint32_t i, uint32_t phase, float dt, float* ent,
+                                                 GroupRows<G>& sm, uint32_t gmask, int gl, int gbase) {
+    static_assert(3 * kJointWords <= kSlotWords && 3 * kJointRowsMost * kJointWords <= G * kSlotWords, "joint rows");
+    constexpr uint32_t kJoints = uint32_t(G) / 3u;
+    const uint32_t jcnt = d.jdeg[i], jlo = d.jinc_off[i];
+    float* const stage = &sm.r[0][0];
+    auto add_staged = [&](const float* row) {
+#pragma unroll
+        for (int q = 0; q < Owned<G>::E; ++q) {
+            const int e = gl + G * q;
+            if (e >= 27) continue;
+            int ei = 0, ek = 0;
+            if (e < 21) entry_ik(e, ei, ek);
+            ent[q] += e < 21 ? row[6] * row[ei] * row[ek] : row[e - 21] * row[7];
+            if (e < 21 && ei == ek && ei >= 3 && row[11] != 0.0f) ent[q] += row[8 + ei - 3];
+        }
+    };
+    if (phase == 0) {
+        const uint32_t mine = uint32_t(gl) / 3u, axis = uint32_t(gl) % 3u;
+        for (uint32_t k = 0; k < jcnt;) {
+            uint32_t j = 0, rows = 0;
+            JointState js{};
+            if (mine < kJoints && k + mine < jcnt) {
+                j = d.jinc_list[jlo + k + mine];
+                js = d.jstate[j];
+                rows = js.enabled ? js.rows : 0u;
+            }
+            const uint32_t before = __popc(rows & ((1u << (axis * kAxisBits)) - 1u));
+            uint32_t mask = (rows >> (axis * kAxisBits)) & kAxisMask;
+            uint32_t count = __popc(mask), taken = min(kJoints, jcnt - k);
+            uint32_t slot_words = kSlotWords;
+            if (__any_sync(gmask, count > 3u)) {
+                taken = 1;
+                slot_words = kJointRowsMost * kJointWords;
+                if (mine != 0) mask = count = 0;
+            }
+            if (mask) {
+                const Joint& o = d.joints[j];
+                const uint32_t type = o.type;
+                const JointEnds en = load_ends(d, js.dense_a, js.dense_b);
+                const JointOld old = load_joint_old(d.jold + size_t(j) * kOldWords, type);
+                const JointPose pose = joint_pose(o, en.xa, en.qa, en.xb, en.qb);
+                const V3 dir = rotate(pose.frame_a, unit_axis(axis));
+                const bool first = i == js.dense_a;
+                const JointRow* src = d.jrows + size_t(j) * 18 + before;
+                float* out = stage + gl * slot_words;
+                for (uint32_t m = mask; m; m &= m - 1u, ++src, out += kJointWords) {
+                    const unsigned bit = __ffs(m) - 1;
+                    const bool angular = bit >= kRowKinds;
+                    const LaneRow r = lane_row(o, pose, old, dir, axis, angular, angular ? bit - kRowKinds : bit,
+                                               en.dxa, en.dxb, Dual{src->lambda, src->penalty}, dt);
+#pragma unroll
+                    for (int c = 0; c < 6; ++c) out[c] = first ? r.ja.v[c] : r.jb.v[c];
+                    out[6] = r.stiff;
+                    out[7] = r.force;
+                    out[11] = angular ? 0.0f : 1.0f;
+                    if (!angular) {
+                        const V3 curv = lane_curvature(dir, first ? add(pose.error, pose.arm_a) : pose.arm_b, r.force);
+                        out[8] = curv.x;
+                        out[9] = curv.y;
+                        out[10] = curv.z;
+                    }
+                }
+            }
+            __syncwarp(gmask);
+            for (uint32_t l = 0; l < 3u * taken; ++l) {
+                const uint32_t n = __shfl_sync(gmask, count, gbase + int(l));
+                for (uint32_t r = 0; r < n; ++r) add_staged(stage + l * slot_words + r * kJointWords);
+            }
+            __syncwarp(gmask);
+            k += taken;
+        }
+    } else {
+        // Velocity phase: the stored rows (formed by the phase's preparation).
+        for (uint32_t k = 0; k < jcnt; ++k) {
+            const uint32_t j = d.jinc_list[jlo + k];
+            const JointState js = d.jstate[j];
+            if (!js.enabled) continue;
+            const bool first = i == js.dense_a;
+            const Lite A = load_lite(d, js.dense_a), B = load_lite(d, js.dense_b);
+            for (uint32_t base = 0; base < js.count; base += G) {
+                const uint32_t r = base + uint32_t(gl);
+                bool hard = false;
+                if (r < js.count) {
+                    const Row row = load_row(d.jrows[size_t(j) * 18 + r]);
+                    hard = row.stiffness >= kMaxPenalty;
+                    if (hard) {
+                        // row_accumulate's terms
+                        const float trial = row_trial(row, A.dx, B.dx, dt);
+                        const bool two_sided = row.lower < 0.0f && row.upper > 0.0f;
+                        float* out = stage + gl * kSlotWords;
+#pragma unroll
+                        for (int c = 0; c < 6; ++c) out[c] = first ? row.a.v[c] : row.b.v[c];
+                        out[6] = two_sided || (trial > row.lower && trial < row.upper)
+                                     ? row.dual.penalty + row.damping / dt
+                                     : 0.0f;
+                        out[7] = fclamp(trial, row.lower, row.upper) - row.reference_force;
+                        out[11] = 0.0f;
+                    }
+                }
+                constexpr uint32_t kLanes = G == 32 ? 0xffffffffu : (1u << (G & 31)) - 1u;
+                uint32_t m = (__ballot_sync(gmask, hard) >> gbase) & kLanes;
+                __syncwarp(gmask);
+                for (; m; m &= m - 1u) add_staged(stage + (__ffs(m) - 1) * kSlotWords);
+                __syncwarp(gmask);
+            }
+        }
+    }
+}
+
 __device__ __forceinline__ unsigned long long gtimer() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -509,12 +645,10 @@ __device__ void solve_body_group(const Dev& d, Ahead& ah, uint32_t kn, uint32_t 
         fetch_codes<G>(d, ah, gl);
     }
     mark(0);
+    if constexpr (Joints) joint_rows_lanes<G>(d, i, phase, dt, ent, sm, gmask, gl, gbase);
+    mark(1);
     Blk blk;
     gather_block<G>(ent, blk, gmask, gbase);
-    mark(1);
-    if constexpr (Joints) {
-        if (d.jdeg[i]) joint_rows_shared<G>(d, i, phase, dt, blk, &sm.jblk, sm.jview, gmask, gl);
-    }
     V6 upd;
     if (!block_solve(blk, upd)) return;
     mark(2);
@@ -784,10 +918,8 @@ static __device__ void dual_contact(const Dev& d, uint32_t c, uint2 ab, float dt
     }
 }
 
-// slots: this thread's two body views and joint residual in shared memory
-// (nullptr: local ones, for kernels without the per-thread slots).
-static __device__ void dual_joint(const Dev& d, uint32_t j, uint32_t phase, float dt, Res& res, uint32_t it,
-                                  BodyView* views = nullptr, JointRes* jres = nullptr) {
+// One thread's dual update of a joint.
+static __device__ void dual_joint(const Dev& d, uint32_t j, uint32_t phase, float dt, Res& res, uint32_t it) {
     JointState js = d.jstate[j];
     if (js.count == 0 || !js.enabled) return;
     const uint32_t a = js.dense_a, b = js.dense_b;
@@ -802,19 +934,13 @@ static __device__ void dual_joint(const Dev& d, uint32_t j, uint32_t phase, floa
     }
     float impulse = 0.0f;
     if (phase == 0) {
-        BodyView local_views[2];
-        JointRes local_res;
-        BodyView* v = views ? views : local_views;
-        JointRes* out = jres ? jres : &local_res;
-        v[0] = load_body(d, a);
-        v[1] = load_body(d, b);
-        *out = JointRes{0.0, 0u, 0.0f, 0u};
+        const BodyView va = load_body(d, a), vb = load_body(d, b);
+        JointRes jr{0.0, 0u, 0.0f, 0u};
         // An advance visit leaves the block alone (no block pointer).
-        impulse = visit_joint(d.joints[j], d.jrows + size_t(j) * 18, v[0], v[1], v3(d.x[a]), q4(d.q[a]), v3(d.x[b]),
-                              q4(d.q[b]), d.p0[a], d.p0[b], dt, nullptr, true, kVisitAdvance, nullptr, out, res.tol);
+        impulse = visit_joint(d.joints[j], d.jrows + size_t(j) * 18, va, vb, v3(d.x[a]), q4(d.q[a]), v3(d.x[b]),
+                              q4(d.q[b]), d.p0[a], d.p0[b], dt, nullptr, true, kVisitAdvance, nullptr, &jr, res.tol);
         // The joint's own residual (a batched world also needs it per scene),
         // added in the same order as a running sum would.
-        const JointRes jr = *out;
         res.sq += jr.sq;
         res.n += jr.n;
         res.mx = fmx(res.mx, jr.mx);
@@ -836,6 +962,98 @@ static __device__ void dual_joint(const Dev& d, uint32_t j, uint32_t phase, floa
     js.applied = impulse;
     const float thr = d.joints[j].breaking_threshold;
     if (thr > 0.0f && impulse > thr) {
+        js.broken = 1;
+        js.enabled = 0;
+    }
+    d.jstate[j] = js;
+}
+
+// dual_joint's position phase by four lanes: lane l < 3 of the quad takes
+// axis l; the sums over the joint's rows (impulse, residual) run through the
+// lanes in row order. Of a row, only its dual changes from sweep to sweep (the
+// rest is formed anew by every visit), so only that is stored. All four lanes
+// call it, with the same j.
+static __device__ __forceinline__ void dual_joint_quad(const Dev& d, uint32_t j, float dt, Res& res, uint32_t it,
+                                                       uint32_t axis, uint32_t qmask, int qbase) {
+    JointState js = d.jstate[j];
+    if (js.count == 0 || !js.enabled) return;
+    const uint32_t a = js.dense_a, b = js.dense_b;
+    uint32_t scene = 0;
+    bool scene_last = false;
+    if (batched(d)) {
+        scene = d.scene_of[a];
+        const uint32_t budget = d.scene_budget[scene];
+        if (it >= budget) return;
+        scene_last = it + 1 == budget;
+    }
+    const Joint& o = d.joints[j];
+    float impulse[kJointRowsMost], viol[kJointRowsMost];
+    uint32_t count = 0;
+    {
+        const uint32_t mask = axis < 3 ? (js.rows >> (axis * kAxisBits)) & kAxisMask : 0u;
+        const uint32_t before = __popc(js.rows & ((1u << (axis * kAxisBits)) - 1u));
+        count = __popc(mask);
+        if (mask) {
+            const JointEnds en = load_ends(d, a, b);
+            const JointOld old = load_joint_old(d.jold + size_t(j) * kOldWords, o.type);
+            const JointPose pose = joint_pose(o, en.xa, en.qa, en.xb, en.qb);
+            const V3 dir = rotate(pose.frame_a, unit_axis(axis));
+            uint32_t m = mask;
+#pragma unroll
+            for (int r = 0; r < kJointRowsMost; ++r) {
+                impulse[r] = viol[r] = 0.0f;
+                if (!m) continue;
+                const unsigned bit = __ffs(m) - 1;
+                m &= m - 1u;
+                const bool angular = bit >= kRowKinds;
+                JointRow& s = d.jrows[size_t(j) * 18 + before + r];
+                const Dual dual{s.lambda, s.penalty};
+                const LaneRow row = lane_row(o, pose, old, dir, axis, angular, angular ? bit - kRowKinds : bit, en.dxa,
+                                             en.dxb, dual, dt);
+                impulse[r] = fab(row.force) * dt;
+                viol[r] = row.stiffness >= kMaxPenalty ? fab(row.error) : -1.0f;  // -1: no hard row
+                const Dual next = update_dual(dual, row.error, s.beta, row.lower, row.upper, row.stiffness);
+                s.lambda = next.lambda;
+                s.penalty = next.penalty;
+            }
+        }
+    }
+    float sum = 0.0f;
+    JointRes jr{0.0, 0u, 0.0f, 0u};
+#pragma unroll
+    for (uint32_t l = 0; l < 3; ++l) {
+        if (axis == l)
+#pragma unroll
+            for (int r = 0; r < kJointRowsMost; ++r)
+                if (r < int(count)) {
+                    sum += impulse[r];
+                    const float v = viol[r];
+                    if (!(v < 0.0f)) {
+                        jr.sq += double(v) * double(v);
+                        jr.n += 1;
+                        jr.mx = fmx(jr.mx, v);
+                        if (v > res.tol) jr.over += 1;
+                    }
+                }
+        sum = __shfl_sync(qmask, sum, qbase + int(l));
+        jr.sq = __shfl_sync(qmask, jr.sq, qbase + int(l));
+        jr.n = __shfl_sync(qmask, jr.n, qbase + int(l));
+        jr.mx = __shfl_sync(qmask, jr.mx, qbase + int(l));
+        jr.over = __shfl_sync(qmask, jr.over, qbase + int(l));
+    }
+    if (axis != 0) return;
+    res.sq += jr.sq;
+    res.n += jr.n;
+    res.mx = fmx(res.mx, jr.mx);
+    res.over += jr.over;
+    if (scene_last && jr.n) {
+        atomicAdd(&d.scene_res_sq[scene], float(jr.sq));
+        atomicAdd(&d.scene_res_n[scene], jr.n);
+        atomicMax(reinterpret_cast<int*>(&d.scene_res_mx[scene]), __float_as_int(fmx(jr.mx, 0.0f)));
+    }
+    js.applied = sum;
+    const float thr = o.breaking_threshold;
+    if (thr > 0.0f && sum > thr) {
         js.broken = 1;
         js.enabled = 0;
     }

@@ -191,10 +191,14 @@ __global__ void __launch_bounds__(T, 1) k_solve(Dev d, StepParams sp, uint32_t p
             }
         }
         if constexpr (kJoints) {
-            BodyView* views = reinterpret_cast<BodyView*>(warp_stage + kThreadViews) + 2 * lane;
-            JointRes* jres = reinterpret_cast<JointRes*>(warp_stage + kThreadJointRes) + lane;
-            for (uint32_t j = grid_stride_begin(); j < d.nj; j += grid_stride())
-                dual_joint(d, j, phase, dt, res, it, views, jres);
+            if (phase == 0) {
+                const int qbase = lane & ~3;
+                for (uint32_t j = grid_stride_begin() / 4u; j < d.nj; j += grid_stride() / 4u)
+                    dual_joint_quad(d, j, dt, res, it, uint32_t(lane & 3), 0xfu << qbase, qbase);
+            } else {
+                for (uint32_t j = grid_stride_begin(); j < d.nj; j += grid_stride())
+                    dual_joint(d, j, phase, dt, res, it);
+            }
         }
         // Deterministic reduction: warp tree, warps in order, blocks in order.
         block_residual<kSolveThreads>(res, wsq, wn, wmx, wov, c, blockIdx.x);

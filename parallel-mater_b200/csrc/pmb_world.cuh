@@ -129,7 +129,9 @@ struct Joint {
 static_assert(sizeof(Joint) == 220, "joint record");
 
 struct JointState {
-    uint32_t enabled, broken, count, dense_a, dense_b, pad0, pad1, pad2;
+    uint32_t enabled, broken, count, dense_a, dense_b;
+    uint32_t rows;  // its rows as bits (joint_row_mask), of an enabled joint
+    uint32_t pad1, pad2;
     float applied;
 };
 
@@ -271,6 +273,7 @@ struct Dev {
     Joint* joints;
     JointState* jstate;
     JointRow* jrows;  // 18 per joint
+    float4* jold;     // 4 per joint: its values at the tick's start (store_joint_old)
     uint32_t* dis_keys;    // sorted (min<<32|max) keys of collision-disabling joints
     uint32_t* dis_joint;   // the joint of each key (a pair may have several)
     uint32_t n_dis;
