@@ -329,7 +329,7 @@ int allocate_world(pmb_world* w, Dev& d, const Sizes& z, Extra& e) {
     ALLOC(d.mp_leaf_off, cap_pair + 1); ALLOC(d.mp_item_off, cap_pair + 1);
     ALLOC(d.ml_rec, cap_contact); ALLOC(d.ml_item, cap_contact); ALLOC(d.ml_pair, cap_contact);
     ALLOC(d.mi_valid, cap_contact); ALLOC(d.mi_p, cap_contact); ALLOC(d.mi_n, cap_contact);
-    ALLOC(d.dxl, n); ALLOC(d.dxa, n); ALLOC(d.dq, n); ALLOC(d.inA, n); ALLOC(d.inB, n);
+    ALLOC(d.dx, 2 * size_t(n)); ALLOC(d.dq, n); ALLOC(d.inA, n); ALLOC(d.inB, n);
     ALLOCS(d.prev_vel, n); ALLOCS(d.color, n);
     ALLOC(d.parent, n); ALLOC(d.impact, n); ALLOC(d.anchored, n); ALLOC(d.mean, n); ALLOC(d.island_end, n);
     ALLOC(d.lo, n); ALLOC(d.hi, n); ALLOC(d.is_large, n); ALLOC(d.large_list, n);
@@ -342,11 +342,10 @@ int allocate_world(pmb_world* w, Dev& d, const Sizes& z, Extra& e) {
     ALLOC(d.st_n, cap_contact); ALLOC(d.st_p, cap_contact);
     ALLOC(d.act_a, cap_pair); ALLOC(d.act_b, cap_pair); ALLOC(d.act_code, cap_pair);
     ALLOC(d.act_off, cap_pair + 1); ALLOC(d.act_cnt, cap_pair); ALLOC(d.act_impact, cap_pair);
-    ALLOC(d.c_pair, cap_contact); ALLOC(d.c_bodies, cap_contact); ALLOC(d.c_jac, 9 * cap_contact);
+    ALLOC(d.c_pair, cap_contact); ALLOC(d.c_bodies, cap_contact); ALLOC(d.c_row, 8 * cap_contact);
     ALLOC(d.c_n, cap_contact); ALLOC(d.c_p, cap_contact); ALLOC(d.c_e, cap_contact);
     ALLOC(d.c_aa, cap_contact); ALLOC(d.c_ab, cap_contact); ALLOC(d.c_lam, cap_contact);
     ALLOC(d.c_pen, cap_contact); ALLOC(d.c_accf, cap_contact); ALLOC(d.c_foff, cap_contact);
-    ALLOC(d.c_mub, cap_contact);
     for (int side = 0; side < 2; ++side) {
         uint64_t** code = side ? &d.out_code : &d.sv_code;
         uint32_t** off = side ? &d.out_off : &d.sv_off;

@@ -37,7 +37,7 @@ __global__ void k_prepare_bodies(Dev d, StepParams sp) {
         d.island_end[i] = 0;
         d.mean[i] = make_float4(0, 0, 0, 0);
         d.dq[i] = make_float4(0, 0, 0, 1);
-        d.dxa[i] = make_float4(0, 0, 0, 0);
+        d.dx[2 * i + 1] = make_float4(0, 0, 0, 0);
         d.deg[i] = 0;
         d.jdeg[i] = 0;
         d.inc_cursor[i] = 0;
@@ -46,7 +46,7 @@ __global__ void k_prepare_bodies(Dev d, StepParams sp) {
         if (d.motion[i] != kDynamic) {
             d.color[i] = kInvalid;
             d.prev_vel[i] = make_float4(0, 0, 0, 0);
-            d.dxl[i] = make_float4(0, 0, 0, 0);
+            d.dx[2 * i] = make_float4(0, 0, 0, 0);
             d.inA[i] = make_float4(0, 0, 0, 0);
             d.inB[i] = make_float4(0, 0, 0, 0);
             continue;
@@ -58,7 +58,7 @@ __global__ void k_prepare_bodies(Dev d, StepParams sp) {
         float wgt = hist && g2 > 0.0f ? fclamp(dot(acc, g) / g2, 0.0f, 1.0f) : 0.0f;
         if (!isfinite(wgt)) wgt = 0.0f;
         V3 corr = mul(g, -(1.0f - wgt) * dt * dt);
-        d.dxl[i] = f4(corr);
+        d.dx[2 * i] = f4(corr);
         d.prev_vel[i] = f4(vprev, 1.0f);
         const float4 p0 = d.p0[i];
         const float mass = 1.0f / fmx(p0.x, 1.0e-12f);

@@ -14,36 +14,25 @@
 
 namespace pmb {
 
-// The position phase also forms each contact's friction and penalty growth
-// factor (c_mub, from its bodies' materials and masses); the velocity phase
-// its force offsets (the row forces are the projected trial forces less
+// Each contact's phase record (d.c_row); its friction and penalty growth
+// factor come from the bodies' materials and masses. The velocity phase also
+// forms the force offsets (the row forces are the projected trial forces less
 // them): the normal impulse and the accumulated friction of the position
-// phase, both fixed by then (k_contact_finalize), over dt.
+// phase, both fixed by then (k_contact_finalize), over dt; its errors are
+// filled in by k_impact_constraints.
 __global__ void k_contact_jacobians(Dev d, uint32_t phase, float dt) {
     if (phase != 0 && d.ctr->impact == 0) return;
     const uint32_t n_con = d.ctr->n_contacts;
     for (uint32_t c = grid_stride_begin(); c < n_con; c += grid_stride()) {
         const uint2 ab = d.c_bodies[c];
+        const uint32_t a = ab.x, b = ab.y;
         V6 ja[3], jb[3];
-        contact_jacobians(v3(d.c_n[c]), v3(d.c_p[c]), v3(d.c_aa[c]), v3(d.c_ab[c]), v3(d.tx[ab.x]), q4(d.tq[ab.x]),
-                          v3(d.tx[ab.y]), q4(d.tq[ab.y]), ja, jb);
-        float f[36];
-#pragma unroll
-        for (int r = 0; r < 3; ++r)
-#pragma unroll
-            for (int k = 0; k < 6; ++k) {
-                f[6 * r + k] = ja[r].v[k];
-                f[18 + 6 * r + k] = jb[r].v[k];
-            }
-        float4* p = d.c_jac + size_t(c) * 9;
-#pragma unroll
-        for (int k = 0; k < 9; ++k) p[k] = make_float4(f[4 * k], f[4 * k + 1], f[4 * k + 2], f[4 * k + 3]);
-        if (phase == 0) {
-            const uint32_t a = ab.x, b = ab.y;
-            const float friction = sqrtf(d.p1[a].x * d.p1[b].x);
-            const float beta = (1.0f / (fmx(d.p0[a].x + d.p0[b].x, 1.0e-6f) * dt * dt)) * 100.0f;
-            d.c_mub[c] = make_float2(friction, beta);
-        } else {
+        contact_jacobians(v3(d.c_n[c]), v3(d.c_p[c]), v3(d.c_aa[c]), v3(d.c_ab[c]), v3(d.tx[a]), q4(d.tq[a]),
+                          v3(d.tx[b]), q4(d.tq[b]), ja, jb);
+        const float friction = sqrtf(d.p1[a].x * d.p1[b].x);
+        const float beta = (1.0f / (fmx(d.p0[a].x + d.p0[b].x, 1.0e-6f) * dt * dt)) * 100.0f;
+        store_row32(d, c, ja, jb, friction, beta, d.c_e[c]);
+        if (phase != 0) {
             V3 t0, t1;
             basis(v3(d.c_n[c]), t0, t1);
             const V3 af = v3(d.c_accf[c]);
@@ -141,12 +130,16 @@ __device__ __forceinline__ void stage_row(const Dev& d, const StageTables& tb, u
     for (int k = 0; k < 6; ++k) me.v[k] = tb.dx[6 * sl + k];
     const Lite o = load_lite(d, other);
     const uint32_t ocol = d.color[other];
-    const float4 lam = d.c_lam[c], pen = d.c_pen[c], e = d.c_e[c];
+    const float4 lam = d.c_lam[c], pen = d.c_pen[c];
+    const ContactRow cr = load_row32(d, c);
+    const float friction = cr.friction, beta = cr.beta;
     V6 ja[3], jb[3];
-    load_jac(d, c, ja, jb);
-    const float2 mub = d.c_mub[c];
-    const float friction = mub.x, beta = mub.y;
-    const float e3[3] = {e.x, e.y, e.z};
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        ja[k] = cr.ja(k);
+        jb[k] = cr.jb(k);
+    }
+    const float* e3 = cr.e;
     float err[3], pre[3], post[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -277,6 +270,63 @@ __device__ void owned_joint_duals(const Dev& d, uint32_t i, uint32_t col, float 
         if (!(ocol == kInvalid || ocol < col)) continue;
         dual_joint(d, j, phase, dt, res, it);
     }
+}
+
+// The group's block in every lane's registers, and back to the lanes' entries.
+template <int G>
+__device__ __forceinline__ void gather_block(const float* ent, Blk& blk, uint32_t gmask, int gbase) {
+#pragma unroll
+    for (int e = 0; e < 21; ++e) blk.h[e] = __shfl_sync(gmask, ent[e / G], gbase + (e % G));
+#pragma unroll
+    for (int r = 0; r < 6; ++r) blk.g[r] = __shfl_sync(gmask, ent[(21 + r) / G], gbase + ((21 + r) % G));
+}
+template <int G> __device__ __forceinline__ void own_entries(const Blk& blk, int gl, float* ent) {
+#pragma unroll
+    for (int m = 0; m < Owned<G>::E; ++m) {
+        const int e = gl + G * m;
+        float v = 0.0f;
+#pragma unroll
+        for (int q = 0; q < 21; ++q) v = e == q ? blk.h[q] : v;
+#pragma unroll
+        for (int r = 0; r < 6; ++r) v = e == 21 + r ? blk.g[r] : v;
+        ent[m] = v;
+    }
+}
+
+// Joint rows of body i added to its block (geometry_constraints_solve.slang:
+// 381-400, the serial loop's order). The joint visit takes the block's
+// address, so lane 0 works on a copy in the group's shared-memory slot `sb`
+// and the group reads the result back: the register block never needs an
+// address (which would put it in local memory for every body).
+template <int G>
+__device__ __forceinline__ void joint_rows_shared(const Dev& d, uint32_t i, uint32_t phase, float dt, Blk& blk,
+                                                  Blk* sb, BodyView* views, uint32_t gmask, int gl) {
+    if (gl == 0) {
+        *sb = blk;
+        const uint32_t jcnt = d.jdeg[i], jlo = d.jinc_off[i];
+        for (uint32_t k = 0; k < jcnt; ++k) {
+            const uint32_t j = d.jinc_list[jlo + k];
+            const JointState js = d.jstate[j];
+            if (!js.enabled) continue;
+            const uint32_t a = js.dense_a, b = js.dense_b;
+            const bool first = i == a;
+            if (phase == 0) {
+                views[0] = load_body(d, a);
+                views[1] = load_body(d, b);
+                visit_joint(d.joints[j], d.jrows + size_t(j) * 18, views[0], views[1], v3(d.x[a]), q4(d.q[a]),
+                            v3(d.x[b]), q4(d.q[b]), d.p0[a], d.p0[b], dt, sb, first, kVisitAccumulate, nullptr);
+            } else {
+                const Lite A = load_lite(d, a), B = load_lite(d, b);
+                for (uint32_t r = 0; r < js.count; ++r) {
+                    Row row = load_row(d.jrows[size_t(j) * 18 + r]);
+                    if (row.stiffness >= kMaxPenalty) row_accumulate(*sb, row, first, A.dx, B.dx, dt);
+                }
+            }
+        }
+    }
+    __syncwarp(gmask);
+    blk = *sb;
+    __syncwarp(gmask);
 }
 
 template <int G>
@@ -417,7 +467,7 @@ __device__ void staged_body(const Dev& d, const StageTables& tb, uint32_t sl, ui
 template <int G>
 __device__ __forceinline__ V6 staged_update(const Dev& d, uint32_t i, uint32_t phase, const V6& upd, uint32_t gmask,
                                             int gl) {
-    float4 l = d.dxl[i], a = d.dxa[i];
+    float4 l = d.dx[2 * i], a = d.dx[2 * i + 1];
     Q4 rel = q4(d.dq[i]);
     __syncwarp(gmask);
     l.x += upd.v[0];
@@ -433,10 +483,10 @@ __device__ __forceinline__ V6 staged_update(const Dev& d, uint32_t i, uint32_t p
             a = make_float4(2.0f * rel.x, 2.0f * rel.y, 2.0f * rel.z, 0.0f);
         }
         if (gl == 0) {
-            d.dxl[i] = l;
+            d.dx[2 * i] = l;
             if (rotates) {
                 d.dq[i] = f4(rel);
-                d.dxa[i] = a;
+                d.dx[2 * i + 1] = a;
             }
         }
     } else {
@@ -444,8 +494,8 @@ __device__ __forceinline__ V6 staged_update(const Dev& d, uint32_t i, uint32_t p
         a.y += upd.v[4];
         a.z += upd.v[5];
         if (gl == 0) {
-            d.dxl[i] = l;
-            d.dxa[i] = a;
+            d.dx[2 * i] = l;
+            d.dx[2 * i + 1] = a;
         }
     }
     return {{l.x, l.y, l.z, a.x, a.y, a.z}};
@@ -497,7 +547,7 @@ __global__ void __launch_bounds__(T, 1) k_solve_staged(Dev d, StepParams sp, uin
                         cnt = skip ? 0u : d.rcount[i];
                         tb.body[threadIdx.x] = i;
                         tb.skip[threadIdx.x] = skip ? 1u : 0u;
-                        const float4 l = d.dxl[i], a = d.dxa[i];
+                        const float4 l = d.dx[2 * i], a = d.dx[2 * i + 1];
                         float* dx = tb.dx + 6 * threadIdx.x;
                         dx[0] = l.x;
                         dx[1] = l.y;
@@ -734,7 +784,7 @@ __global__ void k_free_mean(Dev d, uint32_t phase) {
             float4 l = make_float4(0, 0, 0, 0);
             if (member) {
                 mass = 1.0f / fmx(d.p0[i].x, 1.0e-12f);
-                l = d.dxl[i];
+                l = d.dx[2 * i];
             }
             uint32_t mask = __ballot_sync(0xffffffffu, member);
             while (mask) {
@@ -755,11 +805,11 @@ __global__ void k_free_subtract(Dev d, uint32_t phase) {
     for (uint32_t i = grid_stride_begin(); i < d.n; i += grid_stride()) {
         if (d.motion[i] != kDynamic || (phase != 0 && d.impact[i] == 0)) continue;
         const float4 m = d.mean[d.parent[i]];
-        float4 l = d.dxl[i];
+        float4 l = d.dx[2 * i];
         l.x -= m.x;
         l.y -= m.y;
         l.z -= m.z;
-        d.dxl[i] = l;
+        d.dx[2 * i] = l;
     }
 }
 
@@ -771,7 +821,7 @@ __global__ void k_apply(Dev d, StepParams sp, uint32_t phase, float4* ox, float4
     for (uint32_t i = grid_stride_begin(); i < d.n; i += grid_stride()) {
         if (d.motion[i] != kDynamic) continue;
         if (phase != 0 && d.impact[i] == 0) continue;
-        const float4 l = d.dxl[i], a = d.dxa[i];
+        const float4 l = d.dx[2 * i], a = d.dx[2 * i + 1];
         const V3 lin = v3(l), rot = v3(a);
         V3 x = v3(d.tx[i]), v = v3(d.tv[i]), w = v3(d.tw[i]);
         Q4 q = q4(d.tq[i]);
@@ -836,10 +886,9 @@ __global__ void k_impact_setup(Dev d, StepParams sp, const float4* ox, const flo
         const Lite A = load_lite(d, a), B = load_lite(d, b);
         for (uint32_t q = d.act_off[i]; q < d.act_off[i] + d.act_cnt[i]; ++q) {
             const float4 n4 = d.c_n[q];
-            V6 ja[3], jb[3];
-            load_jac(d, q, ja, jb);  // normal rows: the phase-0 targets' arms
+            const ContactRow cr = load_row32(d, q);  // normal rows: the phase-0 targets' arms
             float4 e = d.c_e[q];
-            e.x = fmx(0.0f, -(n4.w + dot6(ja[0], A.dx) + dot6(jb[0], B.dx)));
+            e.x = fmx(0.0f, -(n4.w + dot6(cr.ja(0), A.dx) + dot6(cr.jb(0), B.dx)));
             d.c_e[q] = e;
         }
     }
@@ -852,8 +901,8 @@ __global__ void k_impact_bodies(Dev d, const float4* ox, const float4* oq, const
             d.tq[i] = oq[i];
             d.tv[i] = ov[i];
             d.tw[i] = ow[i];
-            d.dxl[i] = make_float4(0, 0, 0, 0);
-            d.dxa[i] = make_float4(0, 0, 0, 0);
+            d.dx[2 * i] = make_float4(0, 0, 0, 0);
+            d.dx[2 * i + 1] = make_float4(0, 0, 0, 0);
             d.dq[i] = make_float4(0, 0, 0, 1);
         }
     }
@@ -881,15 +930,16 @@ __global__ void k_impact_constraints(Dev d, StepParams sp, const float4* ov, con
         for (uint32_t q = d.act_off[i]; q < d.act_off[i] + d.act_cnt[i]; ++q) {
             float4 e = d.c_e[q];
             const float gap = e.x;
-            V6 ja[3], jb[3];
-            load_jac(d, q, ja, jb);  // recomputed from the reset targets
+            const ContactRow cr = load_row32(d, q);  // recomputed from the reset targets
             const bool cached = d.c_aa[q].w != 0.0f;
             const float speed = e.w;
             const float rest = !cached && speed < -1.0f ? rest_ab : 0.0f;
-            e.x = dot6(ja[0], va) + dot6(jb[0], vb) - gap - rest * speed * dt;
-            e.y = dot6(ja[1], va) + dot6(jb[1], vb);
-            e.z = dot6(ja[2], va) + dot6(jb[2], vb);
+            e.x = dot6(cr.ja(0), va) + dot6(cr.jb(0), vb) - gap - rest * speed * dt;
+            e.y = dot6(cr.ja(1), va) + dot6(cr.jb(1), vb);
+            e.z = dot6(cr.ja(2), va) + dot6(cr.jb(2), vb);
             d.c_e[q] = e;
+            // The record's errors (its last float4: growth factor, errors).
+            d.c_row[size_t(q) * 8 + 7] = make_float4(cr.beta, e.x, e.y, e.z);
         }
     }
 }

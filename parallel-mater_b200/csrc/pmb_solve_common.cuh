@@ -13,14 +13,14 @@ struct Lite {  // what a contact row needs of a body during the solve: its displ
     V6 dx;
 };
 __device__ __forceinline__ Lite load_lite(const Dev& d, uint32_t i) {
-    const float4 l = d.dxl[i], a = d.dxa[i];
+    const float4 l = d.dx[2 * i], a = d.dx[2 * i + 1];
     return {{{l.x, l.y, l.z, a.x, a.y, a.z}}};
 }
 
 // Contact jacobians (geometry_constraints.slang:508-532). They depend only on
 // the contact geometry and the AVBD target poses, both fixed during a solve
 // phase, so they are evaluated once per phase (k_contact_jacobians) and
-// stored: 36 floats per contact, rows n, t0, t1 for body a then body b.
+// stored in the contact's phase record (d.c_row).
 __device__ __forceinline__ void contact_jacobians(V3 n, V3 pt, V3 anc_a, V3 anc_b, V3 xa, Q4 qa, V3 xb, Q4 qb,
                                                   V6 ja[3], V6 jb[3]) {
     V3 t0, t1;
@@ -36,38 +36,71 @@ __device__ __forceinline__ void contact_jacobians(V3 n, V3 pt, V3 anc_a, V3 anc_
         jb[k] = jac(axes[k], cross(rb, axes[k]));
     }
 }
-__device__ __forceinline__ void load_jac(const Dev& d, uint32_t c, V6 ja[3], V6 jb[3]) {
-    const float4* p = d.c_jac + size_t(c) * 9;
-    float f[36];
+// A contact's phase record (d.c_row): the row values are those of
+// contact_jacobians, with body a's linear parts (the negated axes) not kept.
+struct ContactRow {
+    V3 axis[3], ang_a[3], ang_b[3];
+    float friction, beta;
+    float e[3];
+    __device__ __forceinline__ V6 ja(int k) const {
+        return jac(V3{-axis[k].x, -axis[k].y, -axis[k].z}, ang_a[k]);
+    }
+    __device__ __forceinline__ V6 jb(int k) const { return jac(axis[k], ang_b[k]); }
+};
+__device__ __forceinline__ ContactRow load_row32(const Dev& d, uint32_t c) {
+    const float4* p = d.c_row + size_t(c) * 8;
+    float f[32];
 #pragma unroll
-    for (int k = 0; k < 9; ++k) {
+    for (int k = 0; k < 8; ++k) {
         const float4 v = p[k];
         f[4 * k] = v.x;
         f[4 * k + 1] = v.y;
         f[4 * k + 2] = v.z;
         f[4 * k + 3] = v.w;
     }
+    ContactRow r;
 #pragma unroll
-    for (int r = 0; r < 3; ++r)
-#pragma unroll
-        for (int k = 0; k < 6; ++k) {
-            ja[r].v[k] = f[6 * r + k];
-            jb[r].v[k] = f[18 + 6 * r + k];
-        }
+    for (int k = 0; k < 3; ++k) {
+        r.axis[k] = V3{f[3 * k], f[3 * k + 1], f[3 * k + 2]};
+        r.ang_a[k] = V3{f[9 + 3 * k], f[10 + 3 * k], f[11 + 3 * k]};
+        r.ang_b[k] = V3{f[18 + 3 * k], f[19 + 3 * k], f[20 + 3 * k]};
+        r.e[k] = f[29 + k];
+    }
+    r.friction = f[27];
+    r.beta = f[28];
+    return r;
 }
-__device__ __forceinline__ void contact_rows(const Dev& d, uint32_t c, float4 e, const Lite& A, const Lite& B,
-                                             V6 ja[3], V6 jb[3], float err[3]) {
-    load_jac(d, c, ja, jb);
-    const float e3[3] = {e.x, e.y, e.z};
+__device__ __forceinline__ void store_row32(const Dev& d, uint32_t c, const V6 ja[3], const V6 jb[3], float friction,
+                                            float beta, float4 e) {
+    float f[32];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) err[k] = e3[k] + dot6(ja[k], A.dx) + dot6(jb[k], B.dx);
+    for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            f[3 * k + q] = jb[k].v[q];
+            f[9 + 3 * k + q] = ja[k].v[3 + q];
+            f[18 + 3 * k + q] = jb[k].v[3 + q];
+        }
+    f[27] = friction;
+    f[28] = beta;
+    f[29] = e.x;
+    f[30] = e.y;
+    f[31] = e.z;
+    float4* p = d.c_row + size_t(c) * 8;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) p[k] = make_float4(f[4 * k], f[4 * k + 1], f[4 * k + 2], f[4 * k + 3]);
+}
+// The rows' errors at the bodies' displacements: e + J_a . dx_a + J_b . dx_b.
+__device__ __forceinline__ void contact_errors(const ContactRow& r, const Lite& A, const Lite& B, float err[3]) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) err[k] = r.e[k] + dot6(r.ja(k), A.dx) + dot6(r.jb(k), B.dx);
 }
 
 __device__ __forceinline__ void apply_pose_update(const Dev& d, uint32_t i, const V6& u, float4 l, float4 dq) {
     l.x += u.v[0];
     l.y += u.v[1];
     l.z += u.v[2];
-    d.dxl[i] = l;
+    d.dx[2 * i] = l;
     V3 r{u.v[3], u.v[4], u.v[5]};
     if (r.x == 0.0f && r.y == 0.0f && r.z == 0.0f) return;
     Q4 rel = q4(dq);
@@ -75,10 +108,10 @@ __device__ __forceinline__ void apply_pose_update(const Dev& d, uint32_t i, cons
     rel = qnormalize(Q4{rel.x + 0.5f * dd.x, rel.y + 0.5f * dd.y, rel.z + 0.5f * dd.z, rel.w + 0.5f * dd.w});
     if (rel.w < 0.0f) rel = {-rel.x, -rel.y, -rel.z, -rel.w};
     d.dq[i] = f4(rel);
-    d.dxa[i] = make_float4(2.0f * rel.x, 2.0f * rel.y, 2.0f * rel.z, 0.0f);
+    d.dx[2 * i + 1] = make_float4(2.0f * rel.x, 2.0f * rel.y, 2.0f * rel.z, 0.0f);
 }
 __device__ __forceinline__ void apply_pose_update(const Dev& d, uint32_t i, const V6& u) {
-    apply_pose_update(d, i, u, d.dxl[i], d.dq[i]);
+    apply_pose_update(d, i, u, d.dx[2 * i], d.dq[i]);
 }
 
 // Group-per-body primal: G lanes (G = 8, 16 or 32) solve one body. Lanes
@@ -98,35 +131,36 @@ __device__ __forceinline__ void apply_pose_update(const Dev& d, uint32_t i, cons
 // rows), and a colour ends when its slowest body does, so wider groups
 // there shorten the critical path.
 //
-// Shared-memory banks: the groups of a warp run in step, so their accesses
-// share instructions. A lane's slot is 43 words (odd) and a normal row 9, so
-// the lanes of a group write to distinct banks modulo 8; groups start 8, 16
-// or 24 banks apart, so the four 8-lane (two 16-lane) groups of a warp
-// neither collide on those writes nor on the row reads of the accumulation
-// (each group reads within a 14-word row).
-constexpr int kRowStride = 14;  // words of one staged row
-constexpr int kSlotWords = 43;  // a lane's three rows (42 words) and a pad word
+// A staged contact holds its three rows side by side, one 16-byte word per
+// jacobian component (its n, t0, t1 values): J[6], the forces, then stiffness
+// x J[6], so an entry takes a contact's three products from two 128-bit loads
+// (A and B of entry_words) where it took six of 32 bits. An 8-lane group at
+// 11 contacts a body: 256 instead of about 400 instructions a chunk.
+//
+// Shared-memory banks: a 128-bit access goes eight lanes at a time, and a
+// lane's slot of 52 words puts eight lanes' writes on distinct banks; a group
+// reads distinct words of one slot. Normal rows (scalar accesses) are 9 words,
+// and groups start 24 (8 lanes) or 16 (16 lanes) banks apart, so the groups of
+// a warp do not collide on them either.
+constexpr int kSlotWords = 52;   // a lane's contact: 13 float4
+constexpr int kSlotForce = 24, kSlotScaled = 28;  // words of the forces and of stiffness x J
 template <int G> struct GroupRowsData {
     // Normal rows kept for the crossing safeguard (rows past them are
     // evaluated again there): 32 for 8-lane groups, 64 for the 16- and
     // 32-lane groups of the heavy bodies (which fit the same staging area).
     static constexpr uint32_t kSlots = G >= 16 ? 64u : 32u;
-    // Chunk being accumulated: per lane slot 3 rows of (jacobian[6],
-    // stiffness, force, stiffness x jacobian[6]); the last six are the
-    // Hessian products' first factors, formed once per row instead of once
-    // per entry.
-    float r[G][kSlotWords];
-    float nrow[kSlots][9];  // normal row: jacobian[6], raw penalty, trial force (and a pad word)
+    float r[G][kSlotWords];  // the chunk being accumulated; the body's block while it is factorised
+    float nrow[kSlots][9];   // normal row: jacobian[6], raw penalty, trial force (and a pad word)
 };
-template <int G> struct GroupRows : GroupRowsData<G> {
+template <int G> struct __align__(16) GroupRows : GroupRowsData<G> {
     // Pads the group to 24 banks mod 32 (8 lanes: bases 0, 24, 16, 8) or 16
     // (16 lanes: bases 0, 16).
     static constexpr int kWords = int(sizeof(GroupRowsData<G>) / 4);
     static constexpr int kTarget = G == 8 ? 24 : G == 16 ? 16 : kWords % 32;
     static constexpr int kPad = (kTarget - kWords % 32 + 32) % 32;
     float pad[kPad == 0 ? 32 : kPad];
-    __device__ __forceinline__ float* row(int slot, int x) { return &this->r[slot][kRowStride * x]; }
-    __device__ __forceinline__ const float* row(int slot, int x) const { return &this->r[slot][kRowStride * x]; }
+    __device__ __forceinline__ float4* slot(int s) { return reinterpret_cast<float4*>(&this->r[s][0]); }
+    __device__ __forceinline__ float* block() { return &this->r[0][0]; }  // 27 entries
 };
 static_assert(sizeof(GroupRows<8>) / 4 % 32 == 24 && sizeof(GroupRows<16>) / 4 % 32 == 16, "group bank offsets");
 // Per-warp staging area: four 8-lane groups, two 16-lane groups or one
@@ -148,73 +182,83 @@ __device__ __forceinline__ void entry_ik(int e, int& i, int& k) {
 template <int G> struct Owned {
     static constexpr int E = (27 + G - 1) / G;
 };
+// The lane's entries and the whole block through the group's shared memory.
 template <int G>
-__device__ __forceinline__ void gather_block(const float* ent, Blk& blk, uint32_t gmask, int gbase) {
+__device__ __forceinline__ void publish_entries(const float* ent, GroupRows<G>& sm, int gl) {
 #pragma unroll
-    for (int e = 0; e < 21; ++e) blk.h[e] = __shfl_sync(gmask, ent[e / G], gbase + (e % G));
-#pragma unroll
-    for (int r = 0; r < 6; ++r) blk.g[r] = __shfl_sync(gmask, ent[(21 + r) / G], gbase + ((21 + r) % G));
+    for (int m = 0; m < Owned<G>::E; ++m)
+        if (gl + G * m < 27) sm.block()[gl + G * m] = ent[m];
 }
-template <int G> __device__ __forceinline__ void own_entries(const Blk& blk, int gl, float* ent) {
+template <int G> __device__ __forceinline__ void own_entries(GroupRows<G>& sm, int gl, float* ent) {
 #pragma unroll
-    for (int m = 0; m < Owned<G>::E; ++m) {
-        const int e = gl + G * m;
-        float v = 0.0f;
+    for (int m = 0; m < Owned<G>::E; ++m) ent[m] = gl + G * m < 27 ? sm.block()[gl + G * m] : 0.0f;
+}
+
+// Word offsets in a staged contact of the two factors of entry e's products
+// (three each: n, t0, t1): stiffness x J_i and J_k of the Hessian entry
+// (i, k), J_r and the force of the gradient entry r.
+__device__ __forceinline__ void entry_words(int e, int& a, int& b) {
+    int i, k;
+    entry_ik(e, i, k);
+    a = e < 21 ? kSlotScaled + 4 * i : e < 27 ? 4 * (e - 21) : 0;
+    b = e < 21 ? 4 * k : kSlotForce;
+}
+template <int G>
+__device__ __forceinline__ void accumulate_chunk(float* ent, int gl, GroupRows<G>& sm, uint32_t m) {
+    const float *pa[Owned<G>::E], *pb[Owned<G>::E];
 #pragma unroll
-        for (int q = 0; q < 21; ++q) v = e == q ? blk.h[q] : v;
+    for (int q = 0; q < Owned<G>::E; ++q) {
+        int a, b;
+        entry_words(gl + G * q, a, b);
+        pa[q] = &sm.r[0][a];
+        pb[q] = &sm.r[0][b];
+    }
+    // A contact's products, then the ordered adds (contacts past m are formed
+    // from the slot's stale values and dropped).
+    auto contact = [&](int t, bool in) {
 #pragma unroll
-        for (int r = 0; r < 6; ++r) v = e == 21 + r ? blk.g[r] : v;
-        ent[m] = v;
+        for (int q = 0; q < Owned<G>::E; ++q) {
+            const float4 a = *reinterpret_cast<const float4*>(pa[q] + kSlotWords * t);
+            const float4 b = *reinterpret_cast<const float4*>(pb[q] + kSlotWords * t);
+            const float p0 = a.x * b.x, p1 = a.y * b.y, p2 = a.z * b.z;
+            if (in) {
+                ent[q] += p0;
+                ent[q] += p1;
+                ent[q] += p2;
+            }
+        }
+    };
+    if (G <= 8) {
+#pragma unroll 2  // (more contacts' loads in flight spill at 512 threads)
+        for (int t = 0; t < G; ++t) contact(t, t < int(m));
+    } else {
+#pragma unroll 1
+        for (int t0 = 0; t0 < int(m); t0 += 4)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) contact(t0 + u, t0 + u < int(m));
     }
 }
 
-template <int G>
-__device__ __forceinline__ void accumulate_chunk(float* ent, int gl, const GroupRows<G>& sm, uint32_t m) {
-    static_assert(G <= 8 || G % 4 == 0, "wide groups take rows four at a time");
-    // Products first (independent, pipelined loads), then the ordered adds.
+// The group's block in every lane's registers (seven 128-bit broadcasts
+// where shuffles took 27). Every lane then factorises it: with a lane per row
+// of the block, exchanging rows by shuffles, the solve took 4.0 us instead of
+// 2.7 in the settled pile's first colour -- half the instructions, but each
+// column waits for a shuffle of the one before.
+template <int G> __device__ __forceinline__ void read_block(GroupRows<G>& sm, Blk& blk) {
+    const float4* p = reinterpret_cast<const float4*>(sm.block());
+    float f[28];
 #pragma unroll
-    for (int q = 0; q < Owned<G>::E; ++q) {
-        const int e = gl + G * q;
-        if (e >= 27) continue;
-        int ei = 0, ek = 0;
-        const bool hess = e < 21;
-        if (hess) entry_ik(e, ei, ek);
-        else ei = e - 21;
-        if (G <= 8) {
-            float prod[G][3];
-#pragma unroll
-            for (int t = 0; t < G; ++t)
-#pragma unroll
-                for (int x = 0; x < 3; ++x) {
-                    const float* row = sm.row(t, x);
-                    prod[t][x] = hess ? row[8 + ei] * row[ek] : row[ei] * row[7];
-                }
-#pragma unroll
-            for (int t = 0; t < G; ++t)
-#pragma unroll
-                for (int x = 0; x < 3; ++x)
-                    if (t < int(m)) ent[q] += prod[t][x];
-        } else {
-            // Four rows' products at a time (their loads in flight together),
-            // then their adds in row order; products of rows past m are
-            // formed from the slot's stale values and dropped.
-            for (int t0 = 0; t0 < int(m); t0 += 4) {
-                float prod[4][3];
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-#pragma unroll
-                    for (int x = 0; x < 3; ++x) {
-                        const float* row = sm.row(t0 + u, x);
-                        prod[u][x] = hess ? row[8 + ei] * row[ek] : row[ei] * row[7];
-                    }
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-#pragma unroll
-                    for (int x = 0; x < 3; ++x)
-                        if (t0 + u < int(m)) ent[q] += prod[u][x];
-            }
-        }
+    for (int k = 0; k < 7; ++k) {
+        const float4 v = p[k];
+        f[4 * k] = v.x;
+        f[4 * k + 1] = v.y;
+        f[4 * k + 2] = v.z;
+        f[4 * k + 3] = v.w;
     }
+#pragma unroll
+    for (int e = 0; e < 21; ++e) blk.h[e] = f[e];
+#pragma unroll
+    for (int r = 0; r < 6; ++r) blk.g[r] = f[21 + r];
 }
 
 // Whether a staged normal row's trial force crosses zero under the update
@@ -254,20 +298,17 @@ struct RawContact {
     uint32_t c;
     bool first;
     Lite other;
-    float2 mub;  // the pair's friction and penalty growth factor
-    float4 lam, pen, e;
-    V6 ja[3], jb[3];
+    float4 lam, pen;
+    ContactRow row;
 };
 __device__ __forceinline__ RawContact load_contact(const Dev& d, uint32_t code, uint32_t other_body) {
     RawContact r;
     r.c = code & 0x7fffffffu;
     r.first = (code >> 31) == 0;
     r.other = load_lite(d, other_body);
-    r.mub = d.c_mub[r.c];
     r.lam = d.c_lam[r.c];
     r.pen = d.c_pen[r.c];
-    r.e = d.c_e[r.c];
-    load_jac(d, r.c, r.ja, r.jb);
+    r.row = load_row32(d, r.c);
     return r;
 }
 
@@ -275,64 +316,53 @@ __device__ __forceinline__ RawContact load_contact(const Dev& d, uint32_t code, 
 // raw penalty and normal trial also go to nrow[nslot].
 template <int G>
 __device__ __forceinline__ void stage_loaded(const Dev& d, const Lite& me, const RawContact& rc,
-                                             uint32_t phase, float dt, GroupRows<G>& sm, int slot, int nslot) {
-    const uint32_t c = rc.c;
+                                             uint32_t phase, GroupRows<G>& sm, int slot, int nslot) {
     const bool first = rc.first;
     const Lite A = first ? me : rc.other;  // values, not run-time references (no local copies)
     const Lite B = first ? rc.other : me;
-    const float friction = rc.mub.x;
     const float4 lam = rc.lam, pen = rc.pen;
-    V6 ja[3], jb[3];
     float err[3];
-    {
-        // contact_rows' error terms, from the loaded jacobians
-        const float e3[3] = {rc.e.x, rc.e.y, rc.e.z};
+    contact_errors(rc.row, A, B, err);
+    const F3 trial{lam.x + pen.x * err[0], lam.y + pen.y * err[1], lam.z + pen.z * err[2]};
+    // This body's jacobians: element by element (a reference chosen at run
+    // time would give the arrays addresses, local memory).
+    V6 j[3];
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            ja[k] = rc.ja[k];
-            jb[k] = rc.jb[k];
-            err[k] = e3[k] + dot6(ja[k], A.dx) + dot6(jb[k], B.dx);
-        }
+    for (int x = 0; x < 3; ++x) {
+        const V6 a = rc.row.ja(x), b = rc.row.jb(x);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) j[x].v[k] = first ? a.v[k] : b.v[k];
     }
-    F3 trial{lam.x + pen.x * err[0], lam.y + pen.y * err[1], lam.z + pen.z * err[2]};
     if (nslot >= 0) {
 #pragma unroll
-        for (int k = 0; k < 6; ++k) sm.nrow[nslot][k] = first ? ja[0].v[k] : jb[0].v[k];
+        for (int k = 0; k < 6; ++k) sm.nrow[nslot][k] = j[0].v[k];
         sm.nrow[nslot][6] = pen.x;
         sm.nrow[nslot][7] = trial.n;
     }
     if (slot < 0) return;
     F3 f, sc;
-    project_with_scales(trial, friction, f, sc);
-    float forces[3] = {f.n, f.t0, f.t1};
+    project_with_scales(trial, rc.row.friction, f, sc);
     if (phase != 0) {
-        const float4 fo = d.c_foff[c];
-        forces[0] = f.n - fo.x;
-        forces[1] = f.t0 - fo.y;
-        forces[2] = f.t1 - fo.z;
+        const float4 fo = d.c_foff[rc.c];
+        f.n -= fo.x;
+        f.t0 -= fo.y;
+        f.t1 -= fo.z;
     }
     const float st[3] = {pen.x * sc.n, pen.y * sc.t0, pen.z * sc.t1};
+    float4* out = sm.slot(slot);
 #pragma unroll
-    for (int x = 0; x < 3; ++x) {
-        // Values selected element by element: a reference chosen at run time
-        // between the two arrays would give them addresses (local memory).
-        V6 row;
+    for (int k = 0; k < 6; ++k) out[k] = make_float4(j[0].v[k], j[1].v[k], j[2].v[k], 0.0f);
+    out[kSlotForce / 4] = make_float4(f.n, f.t0, f.t1, 0.0f);
 #pragma unroll
-        for (int k = 0; k < 6; ++k) row.v[k] = first ? ja[x].v[k] : jb[x].v[k];
-        float* out = sm.row(slot, x);
-#pragma unroll
-        for (int k = 0; k < 6; ++k) out[k] = row.v[k];
-        out[6] = st[x];
-        out[7] = forces[x];
-#pragma unroll
-        for (int k = 0; k < 6; ++k) out[8 + k] = st[x] * row.v[k];  // = (stiffness x J_i), as before
-    }
+    for (int k = 0; k < 6; ++k)
+        out[kSlotScaled / 4 + k] =
+            make_float4(st[0] * j[0].v[k], st[1] * j[1].v[k], st[2] * j[2].v[k], 0.0f);  // (stiffness x J_i)
 }
 template <int G>
 __device__ __forceinline__ void stage_contact(const Dev& d, const Lite& me, uint32_t code,
-                                              uint32_t other_body, uint32_t phase, float dt, GroupRows<G>& sm,
-                                              int slot, int nslot) {
-    stage_loaded<G>(d, me, load_contact(d, code, other_body), phase, dt, sm, slot, nslot);
+                                              uint32_t other_body, uint32_t phase, GroupRows<G>& sm, int slot,
+                                              int nslot) {
+    stage_loaded<G>(d, me, load_contact(d, code, other_body), phase, sm, slot, nslot);
 }
 
 // The body a lane group solves next in its colour, fetched while the current
@@ -360,42 +390,6 @@ __device__ __forceinline__ Ahead fetch_ahead(const Dev& d, uint32_t k, int gl) {
     return a;
 }
 
-// Joint rows of body i added to its block (geometry_constraints_solve.slang:
-// 381-400, the serial loop's order). The joint visit takes the block's
-// address, so lane 0 works on a copy in the group's shared-memory slot `sb`
-// and the group reads the result back: the register block never needs an
-// address (which would put it in local memory for every body).
-template <int G>
-__device__ __forceinline__ void joint_rows_shared(const Dev& d, uint32_t i, uint32_t phase, float dt, Blk& blk,
-                                                  Blk* sb, BodyView* views, uint32_t gmask, int gl) {
-    if (gl == 0) {
-        *sb = blk;
-        const uint32_t jcnt = d.jdeg[i], jlo = d.jinc_off[i];
-        for (uint32_t k = 0; k < jcnt; ++k) {
-            const uint32_t j = d.jinc_list[jlo + k];
-            const JointState js = d.jstate[j];
-            if (!js.enabled) continue;
-            const uint32_t a = js.dense_a, b = js.dense_b;
-            const bool first = i == a;
-            if (phase == 0) {
-                views[0] = load_body(d, a);
-                views[1] = load_body(d, b);
-                visit_joint(d.joints[j], d.jrows + size_t(j) * 18, views[0], views[1], v3(d.x[a]), q4(d.q[a]),
-                            v3(d.x[b]), q4(d.q[b]), d.p0[a], d.p0[b], dt, sb, first, kVisitAccumulate, nullptr);
-            } else {
-                const Lite A = load_lite(d, a), B = load_lite(d, b);
-                for (uint32_t r = 0; r < js.count; ++r) {
-                    Row row = load_row(d.jrows[size_t(j) * 18 + r]);
-                    if (row.stiffness >= kMaxPenalty) row_accumulate(*sb, row, first, A.dx, B.dx, dt);
-                }
-            }
-        }
-    }
-    __syncwarp(gmask);
-    blk = *sb;
-    __syncwarp(gmask);
-}
-
 // The two bodies of a joint as its rows read them during a sweep.
 struct JointEnds {
     V6 dxa, dxb;
@@ -403,7 +397,7 @@ struct JointEnds {
     Q4 qa, qb;
 };
 __device__ __forceinline__ void load_end(const Dev& d, uint32_t i, V6& dx, V3& x, Q4& q) {
-    const float4 tx = d.tx[i], tq = d.tq[i], l = d.dxl[i], a = d.dxa[i], dq = d.dq[i];
+    const float4 tx = d.tx[i], tq = d.tq[i], l = d.dx[2 * i], a = d.dx[2 * i + 1], dq = d.dq[i];
     dx = {{l.x, l.y, l.z, a.x, a.y, a.z}};
     x = add(v3(tx), v3(l));
     q = q4(tq);
@@ -629,7 +623,7 @@ __device__ void solve_body_group(const Dev& d, Ahead& ah, uint32_t kn, uint32_t 
             const int nslot = sidx < GroupRows<G>::kSlots ? int(sidx) : -1;
             const uint32_t code = base == 0 ? code0 : base == uint32_t(G) ? code1 : d.blist[ro + sidx];
             const uint32_t other = base == 0 ? other0 : base == uint32_t(G) ? other1 : d.bother[ro + sidx];
-            stage_contact<G>(d, me, code, other, phase, dt, sm, gl, nslot);
+            stage_contact<G>(d, me, code, other, phase, sm, gl, nslot);
         }
         if (base == 0) init_entries();
         __syncwarp(gmask);
@@ -647,45 +641,54 @@ __device__ void solve_body_group(const Dev& d, Ahead& ah, uint32_t kn, uint32_t 
     mark(0);
     if constexpr (Joints) joint_rows_lanes<G>(d, i, phase, dt, ent, sm, gmask, gl, gbase);
     mark(1);
-    Blk blk;
-    gather_block<G>(ent, blk, gmask, gbase);
-    V6 upd;
-    if (!block_solve(blk, upd)) return;
-    mark(2);
-    // The body's rotation offset, read while the safeguard runs (only this
-    // group writes it in the colour), so the update at the end waits on no
-    // load; its displacement is `me` (read at the start; both w are 0).
-    const float4 dq_start = phase == 0 ? d.dq[i] : make_float4(0.0f, 0.0f, 0.0f, 1.0f);
-    // Crossing safeguard (geometry_constraints_solve.slang:433-475): a
-    // ballot per chunk flags the rows; rows past the kept normal rows are
-    // evaluated again into the slots. (Reloading the entries from the block
-    // keeps them out of registers during the factorisation: keeping them
-    // live instead, when no joint rows changed the block, was slower.)
-    own_entries<G>(blk, gl, ent);
+    // The block's solution, then the crossing safeguard
+    // (geometry_constraints_solve.slang:433-475) -- a ballot per chunk flags
+    // the rows; rows past the kept normal rows are evaluated again into the
+    // slots -- and, with the crossing rows added, the solution again. One loop
+    // for both solutions: the factorisation is the longest code here.
     constexpr uint32_t kSlots = GroupRows<G>::kSlots;
-    constexpr uint32_t kLanes = G == 32 ? 0xffffffffu : (1u << G) - 1u;
-    bool crossing = false;
-    for (uint32_t base = 0; base < rn; base += G) {
-        const uint32_t sidx = base + gl;
-        if (base >= kSlots) {
-            __syncwarp(gmask);  // the slots' previous rows are read
-            if (sidx < rn)
-                stage_contact<G>(d, me, d.blist[ro + sidx], d.bother[ro + sidx], phase, dt, sm, -1,
-                                 int(sidx % kSlots));
-            __syncwarp(gmask);
+    constexpr uint32_t kLanes = G == 32 ? 0xffffffffu : (1u << (G & 31)) - 1u;
+    V6 upd;
+    float4 dq_start = make_float4(0.0f, 0.0f, 0.0f, 1.0f);
+#pragma unroll 1
+    for (int pass = 0;; ++pass) {
+        publish_entries<G>(ent, sm, gl);
+        __syncwarp(gmask);
+        Blk blk;
+        read_block<G>(sm, blk);
+        V6 x;
+        const bool solved = block_solve(blk, x);
+        if (pass != 0) {
+            if (solved) upd = x;
+            break;
         }
-        const bool f = sidx < rn && crosses(sm.nrow[sidx % kSlots], upd);
-        const uint32_t m = (__ballot_sync(gmask, f) >> gbase) & kLanes;
-        if (m) {
-            crossing = true;
-            accumulate_crossing<G>(ent, gl, sm, base % kSlots, min(uint32_t(G), rn - base), m);
+        if (!solved) return;
+        upd = x;
+        mark(2);
+        // The body's rotation offset, read while the safeguard runs (only
+        // this group writes it in the colour), so the update at the end waits
+        // on no load; its displacement is `me` (read at the start; both w
+        // are 0).
+        if (phase == 0) dq_start = d.dq[i];
+        bool crossing = false;
+        for (uint32_t base = 0; base < rn; base += G) {
+            const uint32_t sidx = base + gl;
+            if (base >= kSlots) {
+                __syncwarp(gmask);  // the slots' previous rows are read
+                if (sidx < rn)
+                    stage_contact<G>(d, me, d.blist[ro + sidx], d.bother[ro + sidx], phase, sm, -1, int(sidx % kSlots));
+                __syncwarp(gmask);
+            }
+            const bool f = sidx < rn && crosses(sm.nrow[sidx % kSlots], upd);
+            const uint32_t m = (__ballot_sync(gmask, f) >> gbase) & kLanes;
+            if (m) {
+                if (!crossing) own_entries<G>(sm, gl, ent);
+                crossing = true;
+                accumulate_crossing<G>(ent, gl, sm, base % kSlots, min(uint32_t(G), rn - base), m);
+            }
         }
-    }
-    mark(3);
-    if (crossing) {
-        gather_block<G>(ent, blk, gmask, gbase);
-        V6 safe;
-        if (block_solve(blk, safe)) upd = safe;
+        mark(3);
+        if (!crossing) break;
     }
     mark(4);
     if (trace == 1 && gl == 0) atomicMax(&d.ctr->dbg_rn, rn);
@@ -705,8 +708,8 @@ __device__ void solve_body_group(const Dev& d, Ahead& ah, uint32_t kn, uint32_t 
             a.x += upd.v[3];
             a.y += upd.v[4];
             a.z += upd.v[5];
-            d.dxl[i] = l;
-            d.dxa[i] = a;
+            d.dx[2 * i] = l;
+            d.dx[2 * i + 1] = a;
         }
     }
 }
@@ -717,11 +720,12 @@ __device__ void solve_body_group(const Dev& d, Ahead& ah, uint32_t kn, uint32_t 
 // for colours with far more bodies than the grid has lane groups, where a
 // body per thread finishes the colour in fewer rounds than wider groups.
 // `sb`: this thread's shared-memory block slot for the joint visit.
-__device__ __forceinline__ void load_normal_rows(const Dev& d, uint32_t c, V6& ja, V6& jb) {
-    const float4* p = d.c_jac + size_t(c) * 9;
-    const float4 a0 = p[0], a1 = p[1], b4 = p[4], b5 = p[5];  // floats 0-7 and 16-23
-    ja = {{a0.x, a0.y, a0.z, a0.w, a1.x, a1.y}};
-    jb = {{b4.z, b4.w, b5.x, b5.y, b5.z, b5.w}};
+__device__ __forceinline__ float load_normal_rows(const Dev& d, uint32_t c, V6& ja, V6& jb) {
+    const float* p = reinterpret_cast<const float*>(d.c_row + size_t(c) * 8);
+    const V3 n{p[0], p[1], p[2]};
+    ja = jac(V3{-n.x, -n.y, -n.z}, V3{p[9], p[10], p[11]});
+    jb = jac(n, V3{p[18], p[19], p[20]});
+    return p[29];  // the error at the phase's start
 }
 template <bool Joints>
 __device__ void solve_body_thread(const Dev& d, uint32_t i, uint32_t phase, float dt, Blk* sb, BodyView* views) {
@@ -755,14 +759,13 @@ __device__ void solve_body_thread(const Dev& d, uint32_t i, uint32_t phase, floa
         const bool first = (code >> 31) == 0;
         const Lite other = load_lite(d, other_body);
         const Lite A = first ? me : other, B = first ? other : me;
-        const float friction = d.c_mub[c].x;
         const float4 lam = d.c_lam[c], pen = d.c_pen[c];
-        V6 ja[3], jb[3];
+        const ContactRow cr = load_row32(d, c);
         float err[3];
-        contact_rows(d, c, d.c_e[c], A, B, ja, jb, err);
+        contact_errors(cr, A, B, err);
         const F3 trial{lam.x + pen.x * err[0], lam.y + pen.y * err[1], lam.z + pen.z * err[2]};
         F3 f, sc;
-        project_with_scales(trial, friction, f, sc);
+        project_with_scales(trial, cr.friction, f, sc);
         float forces[3] = {f.n, f.t0, f.t1};
         if (phase != 0) {
             const float4 fo = d.c_foff[c];
@@ -774,8 +777,9 @@ __device__ void solve_body_thread(const Dev& d, uint32_t i, uint32_t phase, floa
 #pragma unroll
         for (int x = 0; x < 3; ++x) {
             V6 row;
+            const V6 ja = cr.ja(x), jb = cr.jb(x);
 #pragma unroll
-            for (int k = 0; k < 6; ++k) row.v[k] = first ? ja[x].v[k] : jb[x].v[k];
+            for (int k = 0; k < 6; ++k) row.v[k] = first ? ja.v[k] : jb.v[k];
             add_row(blk, row, st[x], forces[x]);
         }
     }
@@ -818,8 +822,8 @@ __device__ void solve_body_thread(const Dev& d, uint32_t i, uint32_t phase, floa
         const Lite other = load_lite(d, other_body);
         const Lite A = first ? me : other, B = first ? other : me;
         V6 ja, jb;
-        load_normal_rows(d, c, ja, jb);
-        const float err0 = d.c_e[c].x + dot6(ja, A.dx) + dot6(jb, B.dx);
+        const float e0 = load_normal_rows(d, c, ja, jb);
+        const float err0 = e0 + dot6(ja, A.dx) + dot6(jb, B.dx);
         const float k0 = d.c_pen[c].x;
         const float trial = d.c_lam[c].x + k0 * err0;
         V6 nr;
@@ -837,15 +841,15 @@ __device__ void solve_body_thread(const Dev& d, uint32_t i, uint32_t phase, floa
     if (phase == 0) {
         apply_pose_update(d, i, upd);
     } else {
-        float4 l = d.dxl[i], a = d.dxa[i];
+        float4 l = d.dx[2 * i], a = d.dx[2 * i + 1];
         l.x += upd.v[0];
         l.y += upd.v[1];
         l.z += upd.v[2];
         a.x += upd.v[3];
         a.y += upd.v[4];
         a.z += upd.v[5];
-        d.dxl[i] = l;
-        d.dxa[i] = a;
+        d.dx[2 * i] = l;
+        d.dx[2 * i + 1] = a;
     }
 }
 
@@ -885,12 +889,11 @@ static __device__ void dual_contact(const Dev& d, uint32_t c, uint2 ab, float dt
         scene_last = phase == 0 && it + 1 == budget;  // the tick's residual is the pose phase's
     }
     const Lite A = load_lite(d, a), B = load_lite(d, b);
-    const float2 mub = d.c_mub[c];
-    const float friction = mub.x, beta = mub.y;
     float4 lam = d.c_lam[c], pen = d.c_pen[c];
-    V6 ja[3], jb[3];
+    const ContactRow cr = load_row32(d, c);
+    const float friction = cr.friction, beta = cr.beta;
     float err[3];
-    contact_rows(d, c, d.c_e[c], A, B, ja, jb, err);
+    contact_errors(cr, A, B, err);
     F3 f = project_contact(F3{lam.x + pen.x * err[0], lam.y + pen.y * err[1], lam.z + pen.z * err[2]}, friction);
     const float tx = lam.y + pen.y * err[1];
     const float ty = lam.z + pen.z * err[2];

@@ -209,7 +209,8 @@ struct Dev {
     uint8_t* mi_valid;
     float4 *mi_p, *mi_n;
     // AVBD body state
-    float4 *dxl, *dxa, *dq;
+    float4* dx;  // displacement, 2 per body: linear, angular (one 32-byte sector)
+    float4* dq;
     float4 *inA, *inB;  // inertia block: (m/dt2, h33, h43, h44), (h53, h54, h55, -)
     float4* prev_vel;   // xyz + history flag in w
     uint32_t *color, *parent, *impact, *anchored;
@@ -237,16 +238,19 @@ struct Dev {
     uint64_t* act_code;  // a * N + b in 64 bits (the reference's uint32 code while N <= 65,535)
     uint32_t* c_pair;
     uint2* c_bodies;  // (a, b) of the contact's pair
-    float4* c_jac;    // 9 per contact: jacobian rows n,t0,t1 of body a then body b
+    // What a sweep reads of a contact and never writes, one 128-byte line (8
+    // float4, 32 floats): the axes n, t0, t1 (body b's linear jacobians, and
+    // body a's negated), body a's angular jacobians, body b's, the friction
+    // sqrt(mu_a mu_b), the pair's penalty growth factor 100 / (max(w_a + w_b,
+    // 1e-6) dt^2), and the error at the phase's start. Formed once a phase.
+    // (The six jacobians in full, the errors and the two factors were 176
+    // bytes in three arrays: 11 loads a visit and a working set above L2.)
+    float4* c_row;
     float4 *c_n, *c_p, *c_e, *c_aa, *c_ab, *c_lam, *c_pen, *c_accf;
     // Velocity phase: per contact the force offsets of its rows (lambda.w /
     // dt, and the accumulated friction along each tangent / dt), fixed for
     // the phase and formed once with its jacobians.
     float4* c_foff;
-    // Per contact, fixed for the tick: friction sqrt(mu_a mu_b) and the
-    // penalty growth factor 100 / (max(w_a + w_b, 1e-6) dt^2) of its pair,
-    // formed with the position phase's jacobians.
-    float2* c_mub;
     // contact cache from the previous tick (double-buffered by the host)
     uint64_t* sv_code;
     uint32_t *sv_off, *sv_cnt;
