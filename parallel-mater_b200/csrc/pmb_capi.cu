@@ -158,12 +158,9 @@ StepParams params_from(const pmb_step_desc& s) {
 
 // Also the per-scene sums that the predictor and the large-body lists add to.
 __global__ void k_reset_counters(Dev d) {
-    // bar_gen is left alone: it only ever increases.
     uint32_t* w = reinterpret_cast<uint32_t*>(d.ctr);
     const uint32_t words = sizeof(Counters) / 4;
-    const uint32_t skip = offsetof(Counters, bar_gen) / 4;
-    for (uint32_t i = threadIdx.x; i < words; i += blockDim.x)
-        if (i != skip) w[i] = 0;
+    for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) w[i] = 0;
     if (d.n_scenes > 1)
         for (uint32_t i = threadIdx.x; i <= d.n_scenes; i += blockDim.x) {
             d.scene_large_count[i] = 0;
@@ -171,6 +168,30 @@ __global__ void k_reset_counters(Dev d) {
             d.scene_large_cursor[i] = 0;
             d.scene_hs[i] = 0.0f;
         }
+}
+
+// Blocks of the cooperative kernels. Few bodies need few blocks: a barrier
+// costs more the more blocks arrive (1.1 us of 148, 0.5 of 8), and one block
+// needs none and keeps the world in its L1. Colouring: a block of
+// kColorThreads per as many bodies. Solve: 32 lanes a body, and one block up
+// to kOneBlockBodies bodies. Solve time of both phases, us, by blocks (512
+// threads): 22 bodies 215 with 1, 260 with 4, 334 with 148; 56 bodies 336,
+// 287, 355; 211 bodies 908 with 1, 304 with 16, 362 with 148; 1,006 bodies
+// 802 with 64, 862 with 148; 4,101 bodies 1,003 with 64, 950 with 148.
+// A world with a barrier limit of its own keeps every block, so that the
+// limit has barriers to apply to.
+constexpr uint32_t kOneBlockBodies = 40;
+int color_blocks(const pmb_world* w) {
+    if (w->d.barrier_spins != kDefaultBarrierSpins) return w->coop_color;
+    return std::min(w->coop_color, int(blocks_for(w->d.n, kColorThreads)));
+}
+int solve_blocks(const pmb_world* w) {
+    const uint32_t v = w->d.solve_variant < kSolveVariants ? w->d.solve_variant : 0u;
+    const int all = w->coop_solve[v];
+    if (w->d.barrier_spins != kDefaultBarrierSpins) return all;
+    if (w->d.n <= kOneBlockBodies) return 1;
+    const uint64_t threads = uint64_t(solve_variant(v).threads);
+    return int(std::min<uint64_t>(uint64_t(all), (uint64_t(w->d.n) * 32u + threads - 1u) / threads));
 }
 
 void enqueue_step(pmb_world* w, const StepParams& sp) {
@@ -198,9 +219,9 @@ void enqueue_step(pmb_world* w, const StepParams& sp) {
         launch_mlp_apply(d, mlp.meta, mlp.out, mlp.mode, mlp.gate, s);
     }
     prof_mark(s, "mlp features+inference");
-    launch_graph(d, sp, s, w->coop_color);
+    launch_graph(d, sp, s, color_blocks(w));
     launch_scene_budgets(d, sp, s);
-    launch_solve_all(d, sp, s, w->coop_solve, w->out);
+    launch_solve_all(d, sp, s, solve_blocks(w), w->out);
     set_phase(kPhDomain);
     if (mlp.attached && mlp.train) {
         // Online training on this tick's converged normal rows.

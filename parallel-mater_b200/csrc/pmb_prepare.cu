@@ -425,9 +425,10 @@ __global__ void __launch_bounds__(kColorThreads) k_color(Dev d) {
     // The change counter is read by one thread per block and shared: a read
     // by every thread of the grid per round piles onto one L2 line.
     __shared__ uint32_t s_before, s_after;
+    uint32_t arrivals = 0;  // grid_sync
     for (uint32_t round = 0; round < d.n + 2; ++round) {
         if (threadIdx.x == 0) s_before = ((volatile uint32_t*)&c->changed)[0];
-        if (!grid_sync(c, d.barrier_spins)) return;
+        if (!grid_sync(c, kBarColor, arrivals, d.barrier_spins)) return;
         const uint32_t before = s_before;
         uint8_t* cur = d.cdirty + size_t(round & 1u) * d.n;
         uint8_t* next = d.cdirty + size_t((round + 1u) & 1u) * d.n;
@@ -448,7 +449,7 @@ __global__ void __launch_bounds__(kColorThreads) k_color(Dev d) {
         }
         changes = __reduce_add_sync(0xffffffffu, changes);  // one atomic per warp
         if (changes && (threadIdx.x & 31) == 0) atomicAdd(&c->changed, changes);
-        if (!grid_sync(c, d.barrier_spins)) return;
+        if (!grid_sync(c, kBarColor, arrivals, d.barrier_spins)) return;
         if (threadIdx.x == 0) s_after = ((volatile uint32_t*)&c->changed)[0];
         __syncthreads();
         const uint32_t after = s_after;

@@ -522,6 +522,7 @@ __global__ void __launch_bounds__(T, 1) k_solve_staged(Dev d, StepParams sp, uin
     __shared__ uint32_t wn[T / 32], wov[T / 32];
     __shared__ float wmx[T / 32];
     const bool timing = Timed && phase == 0;
+    uint32_t arrivals = 0;  // grid_sync
     if (timing && blockIdx.x == 0 && threadIdx.x == 0) c->dbg_start = gtimer();
     for (uint32_t it = 0; it < iters; ++it) {
         Res res{0.0, 0u, 0.0f, 0u, sp.tolerance};
@@ -654,11 +655,11 @@ __global__ void __launch_bounds__(T, 1) k_solve_staged(Dev d, StepParams sp, uin
                 // The sweep's residual partials (after the last colour's
                 // duals), published by the barrier below.
                 block_residual<T>(res, wsq, wn, wmx, wov, c, parity + blockIdx.x);
-                if (!grid_sync(c, d.barrier_spins)) return;
+                if (!grid_sync(c, kBarSolve + phase, arrivals, d.barrier_spins)) return;
                 if (timing && it == 0 && col < 19 && blockIdx.x == 0 && threadIdx.x == 0) c->dbg_release[col] = gtimer();
                 break;
             }
-            if (!grid_sync(c, d.barrier_spins)) return;
+            if (!grid_sync(c, kBarSolve + phase, arrivals, d.barrier_spins)) return;
             if (timing && it == 0 && col < 19 && blockIdx.x == 0 && threadIdx.x == 0) c->dbg_release[col] = gtimer();
         }
         const SweepResidual sw = sweep_residual(c, parity, sp);
@@ -1019,10 +1020,10 @@ __global__ void k_contact_events(Dev d) {
     }
 }
 
-void launch_solve_all(const Dev& d, const StepParams& sp, cudaStream_t s, const int* coop_blocks,
+void launch_solve_all(const Dev& d, const StepParams& sp, cudaStream_t s, int coop_blocks,
                       const SolveBuffers& o) {
     const SolveVariant& sv = solve_variant(d.solve_variant);
-    const int coop = coop_blocks[d.solve_variant < kSolveVariants ? d.solve_variant : 0];
+    const int coop = coop_blocks;
     const int feat = solve_features(d);
     const uint32_t pb = cap_blocks(d.cap_pair > d.nj ? d.cap_pair : d.nj);
     for (uint32_t phase = 0; phase < (sp.realtime ? 1u : 2u); ++phase) {

@@ -44,6 +44,7 @@ __global__ void __launch_bounds__(T, 1) k_solve(Dev d, StepParams sp, uint32_t p
     __shared__ uint32_t wn[kSolveThreads / 32], wov[kSolveThreads / 32];
     __shared__ float wmx[kSolveThreads / 32];
     const bool timing = Timed && phase == 0;
+    uint32_t arrivals = 0;  // grid_sync
     auto now = [] {
         unsigned long long t;
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -173,7 +174,7 @@ __global__ void __launch_bounds__(T, 1) k_solve(Dev d, StepParams sp, uint32_t p
                 __syncthreads();
                 if (threadIdx.x == 0) atomicMax(&c->dbg_work[col], now());
             }
-            if (!grid_sync(c, d.barrier_spins)) return;
+            if (!grid_sync(c, kBarSolve + phase, arrivals, d.barrier_spins)) return;
             if (timing && it == 0 && col < 18 && blockIdx.x == 0 && threadIdx.x == 0) c->dbg_release[col] = now();
         }
         Res res{0.0, 0u, 0.0f, 0u, sp.tolerance};
@@ -203,14 +204,14 @@ __global__ void __launch_bounds__(T, 1) k_solve(Dev d, StepParams sp, uint32_t p
         // Deterministic reduction: warp tree, warps in order, blocks in order.
         block_residual<kSolveThreads>(res, wsq, wn, wmx, wov, c, blockIdx.x);
         if (timing && it == 0 && threadIdx.x == 0) atomicMax(&c->dbg_work[19], now());
-        if (!grid_sync(c, d.barrier_spins)) return;
+        if (!grid_sync(c, kBarSolve + phase, arrivals, d.barrier_spins)) return;
         if (timing && it == 0 && blockIdx.x == 0 && threadIdx.x == 0) c->dbg_release[19] = now();
         const SweepResidual sw = sweep_residual(c, 0u, sp);
         if (phase == 0 && grid_stride_begin() == 0) c->residual_trace[it] = sw.measure;
         bool last = it + 1 == iters;
         if (adaptive && sw.met) last = true;
         // Every block has read the partials before the next pass rewrites them.
-        if (!last && colors == 0 && !grid_sync(c, d.barrier_spins)) return;
+        if (!last && colors == 0 && !grid_sync(c, kBarSolve + phase, arrivals, d.barrier_spins)) return;
         if (last) {
             if (grid_stride_begin() == 0) {
                 c->claim[0] = c->claim[1] = 0u;  // every block is past its last claim

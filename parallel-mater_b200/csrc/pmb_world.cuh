@@ -57,7 +57,7 @@ struct Counters {
     uint32_t n_cand, n_stage, n_act, n_contacts;
     uint32_t n_large, colors, islands, iterations;
     uint32_t impact, status, changed, rounds;
-    uint32_t bar_count, bar_gen, budget, joint_iters;
+    uint32_t bar[3], budget, joint_iters;
     float hs, residual, pad1, pad2;
     uint32_t budget_max;  // batched scenes: the largest scene budget of the tick
     uint32_t n_surv;      // narrowphase candidates left for the manifold pass
@@ -301,37 +301,39 @@ struct Dev {
 __device__ __forceinline__ uint32_t grid_stride_begin() { return blockIdx.x * blockDim.x + threadIdx.x; }
 __device__ __forceinline__ uint32_t grid_stride() { return gridDim.x * blockDim.x; }
 
-// Grid barrier for cooperative launches: arrive on a counter, the last block
-// bumps the generation. Waits are bounded by `spins` polls (about 2^26 by
-// default, seconds); a timeout latches kStBarrierTimeout and the caller
-// abandons the tick: every later cooperative kernel of the tick returns at
-// once, and the host reports the status.
+// Grid barrier for cooperative launches: a block arrives on a counter that
+// only grows during the kernel (one per cooperative kernel of the tick,
+// cleared with the tick's counters) and waits until every block's arrival of
+// this barrier is in. One L2 round trip after the last arrival -- where a
+// last block that bumps a generation for the others takes two, and a sleep
+// between polls adds to it: 2.1 us a barrier on 148 blocks then. A
+// grid of one block needs no more than __syncthreads. Waits are bounded by
+// `spins` polls (about 2^26 by default, tens of seconds); a timeout latches
+// kStBarrierTimeout and the caller abandons the tick: every later
+// cooperative kernel of the tick returns at once, and the host reports the
+// status. `target`: this thread's running count of awaited arrivals (0 at the
+// kernel's start).
 constexpr uint32_t kDefaultBarrierSpins = 1u << 26;
-__device__ __forceinline__ bool grid_sync(Counters* c, uint32_t spins_limit) {
+enum : uint32_t { kBarColor = 0, kBarSolve = 1, kBarCount = 3 };  // kBarSolve + phase
+__device__ __forceinline__ bool grid_sync(Counters* c, uint32_t which, uint32_t& target, uint32_t spins_limit) {
     __syncthreads();
+    if (gridDim.x == 1) return true;
     __shared__ int ok;
+    target += gridDim.x;
     if (threadIdx.x == 0) {
         ok = 1;
-        volatile uint32_t* gen = &c->bar_gen;
-        uint32_t g = *gen;
-        __threadfence();
-        uint32_t arrived = atomicAdd(&c->bar_count, 1u);
-        if (arrived == gridDim.x - 1) {
-            c->bar_count = 0;
-            __threadfence();
-            atomicAdd(&c->bar_gen, 1u);
-        } else {
-            uint32_t spins = 0;
-            while (*gen == g) {
-                if (++spins > spins_limit) {
-                    atomicOr(&c->status, kStBarrierTimeout);
-                    ok = 0;
-                    break;
-                }
-                __nanosleep(32);
+        uint32_t* bar = &c->bar[which];
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+        uint32_t seen, spins = 0;
+        for (;;) {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
+            if (int32_t(seen - target) >= 0) break;
+            if (++spins > spins_limit) {
+                atomicOr(&c->status, kStBarrierTimeout);
+                ok = 0;
+                break;
             }
         }
-        __threadfence();
     }
     __syncthreads();
     return ok != 0;
@@ -358,7 +360,7 @@ void launch_prepare(const Dev& d, const StepParams& sp, cudaStream_t s);
 void launch_graph(const Dev& d, const StepParams& sp, cudaStream_t s, int coop_blocks);
 struct SolveBuffers { float4 *ox, *oq, *ov, *ow; };
 void launch_integrate(const Dev& d, const StepParams& sp, cudaStream_t s, const SolveBuffers& o);
-void launch_solve_all(const Dev& d, const StepParams& sp, cudaStream_t s, const int* coop_blocks,
+void launch_solve_all(const Dev& d, const StepParams& sp, cudaStream_t s, int coop_blocks,
                       const SolveBuffers& o);
 void launch_body_constants(const Dev& d, const float4* lo, const float4* hi, const float4* sph, cudaStream_t s);
 void launch_finish(const Dev& d, const StepParams& sp, cudaStream_t s);
