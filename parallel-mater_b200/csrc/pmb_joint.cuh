@@ -24,7 +24,7 @@ __device__ __forceinline__ BodyView load_body(const Dev& d, uint32_t i) {
     BodyView b;
     b.x = v3(d.tx[i]);
     b.q = q4(d.tq[i]);
-    float4 l = d.dxl[i], a = d.dxa[i];
+    float4 l = d.dx[2 * i], a = d.dx[2 * i + 1];
     b.dx = {{l.x, l.y, l.z, a.x, a.y, a.z}};
     b.dq = q4(d.dq[i]);
     b.v = v3(d.tv[i]);
