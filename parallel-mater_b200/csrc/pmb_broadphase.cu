@@ -257,6 +257,58 @@ __global__ void k_grid_scatter(Dev d) {
     }
 }
 
+// Count, scan and scatter by one block, bucket counts in shared memory: up to
+// kOneBlockGrid buckets (half as many bodies), where three launches cost more.
+constexpr uint32_t kOneBlockGrid = 8192;
+__global__ void __launch_bounds__(1024) k_grid_build(Dev d) {
+    __shared__ uint32_t count[kOneBlockGrid];
+    __shared__ uint32_t part[32];
+    constexpr uint32_t kPer = kOneBlockGrid / 1024;
+    const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
+#pragma unroll
+    for (uint32_t k = 0; k < kPer; ++k) count[t + 1024u * k] = 0;
+    __syncthreads();
+    for (uint32_t i = t; i < d.n; i += 1024u) {
+        if (d.is_large[i] != 0) continue;
+        const float h = batched(d) ? d.scene_hs[d.scene_of[i]] : d.ctr->hs;
+        const int4 c = cell_of(d.lo[i], d.hi[i], h > 0.0f ? h : 1.0f);
+        d.grid_cell[i] = c;
+        atomicAdd(&count[cell_bucket(c.x, c.y, c.z, d.grid_size, scene_of(d, i))], 1u);
+    }
+    __syncthreads();
+    // Exclusive scan, kPer consecutive buckets per thread; counts become the
+    // buckets' next slots.
+    uint32_t v[kPer], sum = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < kPer; ++k) {
+        v[k] = count[t * kPer + k];
+        sum += v[k];
+    }
+    uint32_t x = sum;
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= uint32_t(o)) x += y;
+    }
+    if (lane == 31) part[warp] = x;
+    __syncthreads();
+    uint32_t run = x - sum;
+    for (uint32_t w = 0; w < warp; ++w) run += part[w];
+#pragma unroll
+    for (uint32_t k = 0; k < kPer; ++k) {
+        const uint32_t b = t * kPer + k;
+        if (b <= d.grid_size) d.bucket_off[b] = run;
+        count[b] = run;
+        run += v[k];
+    }
+    if (t == 1023 && d.grid_size == kOneBlockGrid) d.bucket_off[kOneBlockGrid] = run;
+    __syncthreads();
+    for (uint32_t i = t; i < d.n; i += 1024u) {
+        if (d.is_large[i] != 0) continue;
+        const int4 c = d.grid_cell[i];
+        d.grid_body[atomicAdd(&count[cell_bucket(c.x, c.y, c.z, d.grid_size, scene_of(d, i))], 1u)] = i;
+    }
+}
+
 __device__ __forceinline__ bool aabb_overlap(float4 alo, float4 ahi, float4 blo, float4 bhi) {
     return ahi.x >= blo.x && ahi.y >= blo.y && ahi.z >= blo.z && bhi.x >= alo.x && bhi.y >= alo.y && bhi.z >= alo.z;
 }
@@ -445,11 +497,16 @@ void launch_broadphase(const Dev& d, cudaStream_t s) {
         k_scene_large_scatter<<<blocks_for(d.n), kBlock, 0, s>>>(d);
         note_launch(blocks_for(d.n));
     }
-    k_grid_count<<<blocks_for(d.n), kBlock, 0, s>>>(d);
-    note_launch(blocks_for(d.n));
-    scan_u32(d.bucket_count, d.bucket_off, nullptr, d.grid_size, nullptr, 0u, d.scan_tmp32, s);
-    k_grid_scatter<<<blocks_for(d.n), kBlock, 0, s>>>(d);
-    note_launch(blocks_for(d.n));
+    if (d.grid_size <= kOneBlockGrid) {
+        k_grid_build<<<1, 1024, 0, s>>>(d);
+        note_launch(1);
+    } else {
+        k_grid_count<<<blocks_for(d.n), kBlock, 0, s>>>(d);
+        note_launch(blocks_for(d.n));
+        scan_u32(d.bucket_count, d.bucket_off, nullptr, d.grid_size, nullptr, 0u, d.scan_tmp32, s);
+        k_grid_scatter<<<blocks_for(d.n), kBlock, 0, s>>>(d);
+        note_launch(blocks_for(d.n));
+    }
     prof_mark(s, "grid build");
     set_phase(kPhCandidates);
     if (d.n_fixed) {

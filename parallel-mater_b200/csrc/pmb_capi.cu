@@ -390,10 +390,10 @@ int allocate_world(pmb_world* w, Dev& d, const Sizes& z, Extra& e) {
     ALLOC(d.jold, size_t(nj) * kOldWords);
     ALLOCP(d.hinge_list, z.hinges); ALLOCP(d.hinge_seg, z.hinge_segs + 1);
     {
-        // Scan scratch: one slot per 2048-element tile of the longest scan plus the total.
+        // Scan scratch: one slot per 2048-element tile of the longest scan (two of them together).
         size_t longest = std::max<size_t>({cap_cand, grid_size, n, cap_pair});
         size_t tiles = (longest + 2047) / 2048 + 2;
-        ALLOC(d.scan_tmp, tiles); ALLOC(d.scan_tmp32, tiles);
+        ALLOC(d.scan_tmp, tiles); ALLOC(d.scan_tmp32, 2 * tiles);
     }
     ALLOCP(d.ctr, 1);
     ALLOC(e.lo, nm); ALLOC(e.hi, nm); ALLOC(e.sph, nm);

@@ -980,8 +980,8 @@ void launch_mesh_narrowphase(const Dev& d, const StepParams& sp, cudaStream_t s)
     k_mesh_walk_count<<<pairs_grid, 128, 0, s>>>(d);
     note_launch(pairs_grid);
     prof_mark(s, "mesh walk");
-    scan_u32(d.mp_leaves, d.mp_leaf_off, &d.ctr->n_mesh, d.cap_mesh, &d.ctr->n_mesh_leaves, 0xffffffffu, d.scan_tmp32, s);
-    scan_u32(d.mp_items, d.mp_item_off, &d.ctr->n_mesh, d.cap_mesh, &d.ctr->n_mesh_items, 0xffffffffu, d.scan_tmp32, s);
+    scan_u32_pair(d.mp_leaves, d.mp_leaf_off, &d.ctr->n_mesh_leaves, d.mp_items, d.mp_item_off, &d.ctr->n_mesh_items,
+                  &d.ctr->n_mesh, d.cap_mesh, d.scan_tmp32, s);
     prof_mark(s, "mesh scans");
     k_mesh_walk_write<<<pairs_grid, 128, 0, s>>>(d);
     note_launch(pairs_grid);

@@ -20,11 +20,13 @@
 //             colours until a round changes nothing: the result equals the
 //             serial colouring exactly, in few rounds when the graph changed
 //             little.
-#include "pmb_joint.cuh"
+#include <algorithm>
+
+#include "pmb_solve_common.cuh"
 
 namespace pmb {
 
-__global__ void k_prepare_bodies(Dev d, StepParams sp) {
+__device__ __forceinline__ void prepare_bodies(const Dev& d, const StepParams& sp) {
     const float dt = sp.dt;
     const V3 g{sp.gx, sp.gy, sp.gz};
     for (uint32_t i = grid_stride_begin(); i < d.n; i += grid_stride()) {
@@ -86,7 +88,7 @@ __device__ __forceinline__ float pair_stiffness(float ima, float imb, float dt) 
 }
 
 // geometry_constraints.slang:1297-1389 and the impact test :983-1006.
-__global__ void k_prepare_pairs(Dev d, StepParams sp) {
+__device__ __forceinline__ void prepare_pairs(const Dev& d, const StepParams& sp) {
     const float dt = sp.dt;
     const bool realtime = sp.realtime != 0;
     const uint32_t n_act = d.ctr->n_act;
@@ -170,6 +172,12 @@ __global__ void k_prepare_pairs(Dev d, StepParams sp) {
     }
 }
 
+// (Pairs read nothing that the bodies' part writes.)
+__global__ void __launch_bounds__(128) k_prepare(Dev d, StepParams sp) {
+    prepare_bodies(d, sp);
+    prepare_pairs(d, sp);
+}
+
 __global__ void k_prepare_joints(Dev d, StepParams sp) {
     const float dt = sp.dt;
     for (uint32_t j = grid_stride_begin(); j < d.nj; j += grid_stride()) {
@@ -228,7 +236,17 @@ __device__ void uf_unite(uint32_t* parent, uint32_t a, uint32_t b) {
     }
 }
 
+// The incidence counts and unions, and each contact's record of the position
+// phase (which only the sweeps read).
 __global__ void k_graph_degrees(Dev d, StepParams sp) {
+    const uint32_t n_con = d.ctr->n_contacts;
+    for (uint32_t c = grid_stride_begin(); c < n_con; c += grid_stride()) {
+        const uint2 ab = d.c_bodies[c];
+        V6 ja[3], jb[3];
+        float friction, beta;
+        contact_phase_row(d, c, ab.x, ab.y, sp.dt, ja, jb, friction, beta);
+        store_row32(d, c, ja, jb, friction, beta, d.c_e[c]);
+    }
     const uint32_t n_act = d.ctr->n_act;
     for (uint32_t i = grid_stride_begin(); i < n_act; i += grid_stride()) {
         const uint32_t a = d.act_a[i], b = d.act_b[i];
@@ -325,7 +343,7 @@ __global__ void k_graph_roots(Dev d) {
 
 // Flattened contact list per body, in the reference's visiting order
 // (incident pairs by descending index, points in manifold order).
-__global__ void k_row_lists(Dev d) {
+__device__ __forceinline__ void row_lists(const Dev& d) {
     for (uint32_t i = grid_stride_begin(); i < d.n; i += grid_stride()) {
         uint32_t pos = d.roff[i];
         const uint32_t lo = d.inc_off[i], n = d.deg[i];
@@ -343,7 +361,7 @@ __global__ void k_row_lists(Dev d) {
     }
 }
 
-__global__ void k_graph_impact(Dev d) {
+__device__ __forceinline__ void graph_impact(const Dev& d) {
     const uint32_t n_act = d.ctr->n_act;
     for (uint32_t i = grid_stride_begin(); i < n_act; i += grid_stride()) {
         if (!d.act_impact[i]) continue;
@@ -353,7 +371,7 @@ __global__ void k_graph_impact(Dev d) {
     }
 }
 
-__global__ void k_graph_islands(Dev d) {
+__device__ __forceinline__ void graph_islands(const Dev& d) {
     for (uint32_t i = grid_stride_begin(); i < d.n; i += grid_stride()) {
         if (d.motion[i] != kDynamic) continue;
         const uint32_t r = d.parent[i];
@@ -381,7 +399,7 @@ __device__ __forceinline__ uint32_t mex_lower(const Dev& d, uint32_t v, bool& ov
 // rounds: lower-indexed ones from the front of its segment (nlow of them),
 // higher-indexed ones from the back (nhigh). Segment base = inc_off + jinc_off
 // (room for deg + jdeg entries).
-__global__ void k_neighbour_lists(Dev d) {
+__device__ __forceinline__ void neighbour_lists(const Dev& d) {
     for (uint32_t v = grid_stride_begin(); v < d.n; v += grid_stride()) {
         if (d.motion[v] != kDynamic) continue;
         const uint32_t base = d.inc_off[v] + d.jinc_off[v], len = d.deg[v] + d.jdeg[v];
@@ -405,6 +423,14 @@ __global__ void k_neighbour_lists(Dev d) {
         d.nlow[v] = lo;
         d.nhigh[v] = hi;
     }
+}
+
+// What the sorted lists and the roots give: contact rows, neighbours, impact
+// marks at the islands' roots.
+__global__ void k_graph_rows(Dev d) {
+    row_lists(d);
+    neighbour_lists(d);
+    graph_impact(d);
 }
 
 // Mark v's higher-indexed dynamic neighbours for the next round: only their
@@ -469,27 +495,28 @@ __global__ void __launch_bounds__(kColorThreads) k_color(Dev d) {
     if (grid_stride_begin() == 0) atomicOr(&c->status, kStColorOverflow);
 }
 
-__global__ void k_color_count(Dev d) {
-    for (uint32_t i = grid_stride_begin(); i < d.n; i += grid_stride()) {
-        if (d.motion[i] != kDynamic) continue;
-        const uint32_t col = d.color[i];
-        atomicAdd(&d.ctr->color_count[col * kSortClasses + sort_class(d.rcount[i])], 1u);
-        atomicMax(&d.ctr->colors, col + 1);
-    }
+__device__ __forceinline__ uint32_t color_bucket(const Dev& d, uint32_t i) {
+    return d.color[i] * kSortClasses + sort_class(d.rcount[i]);
+}
+__device__ __forceinline__ void place_in_order(const Dev& d, uint32_t i, uint32_t slot) {
+    d.corder[slot] = i;
+    d.crec[slot] = make_uint4(i, d.roff[i], d.rcount[i], d.impact[i]);
 }
 
-// Exclusive scan of the bucket counts (one block, kPer consecutive buckets
-// per thread); counts become cursors.
 constexpr uint32_t kBuckets = kMaxColors * kSortClasses;
 constexpr uint32_t kPer = (kBuckets + 1023) / 1024;
-__global__ void __launch_bounds__(1024) k_color_offsets(Dev d) {
+static_assert(kPer * 1024 >= kBuckets, "bucket scan is one block");
+
+// Exclusive scan of the bucket counts by one block (kPer consecutive buckets
+// per thread) into color_off; counts become cursors from zero.
+__device__ __forceinline__ void color_offsets(const Dev& d, uint32_t* count) {
     __shared__ uint32_t part[32];
     const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
     uint32_t v[kPer], sum = 0;
 #pragma unroll
     for (uint32_t k = 0; k < kPer; ++k) {
         const uint32_t b = t * kPer + k;
-        v[k] = b < kBuckets ? d.ctr->color_count[b] : 0u;
+        v[k] = b < kBuckets ? count[b] : 0u;
         sum += v[k];
     }
     uint32_t x = sum;
@@ -514,33 +541,64 @@ __global__ void __launch_bounds__(1024) k_color_offsets(Dev d) {
         const uint32_t b = t * kPer + k;
         if (b < kBuckets) {
             d.ctr->color_off[b] = run;
-            d.ctr->color_count[b] = 0;
+            count[b] = 0;
         }
         run += v[k];
         if (b == kBuckets - 1) d.ctr->color_off[kBuckets] = run;
     }
 }
 
+// Islands, and the bodies in colour order: three launches across the grid,
+// or one block (counts and cursors in shared memory) up to kOneBlockOrder
+// bodies, where the launches cost more than the block's few rounds.
+constexpr uint32_t kOneBlockOrder = 8192;
+__global__ void k_color_count(Dev d) {
+    graph_islands(d);
+    for (uint32_t i = grid_stride_begin(); i < d.n; i += grid_stride()) {
+        if (d.motion[i] != kDynamic) continue;
+        atomicAdd(&d.ctr->color_count[color_bucket(d, i)], 1u);
+        atomicMax(&d.ctr->colors, d.color[i] + 1);
+    }
+}
+__global__ void __launch_bounds__(1024) k_color_offsets(Dev d) { color_offsets(d, d.ctr->color_count); }
 __global__ void k_color_scatter(Dev d) {
     for (uint32_t i = grid_stride_begin(); i < d.n; i += grid_stride()) {
         if (d.motion[i] != kDynamic) continue;
-        const uint32_t b = d.color[i] * kSortClasses + sort_class(d.rcount[i]);
-        const uint32_t slot = d.ctr->color_off[b] + atomicAdd(&d.ctr->color_count[b], 1u);
-        d.corder[slot] = i;
-        d.crec[slot] = make_uint4(i, d.roff[i], d.rcount[i], d.impact[i]);
+        const uint32_t b = color_bucket(d, i);
+        place_in_order(d, i, d.ctr->color_off[b] + atomicAdd(&d.ctr->color_count[b], 1u));
+    }
+}
+__global__ void __launch_bounds__(1024) k_color_order(Dev d) {
+    __shared__ uint32_t count[kBuckets];
+    __shared__ uint32_t colors;
+    for (uint32_t b = threadIdx.x; b < kBuckets; b += blockDim.x) count[b] = 0;
+    if (threadIdx.x == 0) colors = 0;
+    __syncthreads();
+    graph_islands(d);
+    for (uint32_t i = threadIdx.x; i < d.n; i += blockDim.x) {
+        if (d.motion[i] != kDynamic) continue;
+        atomicAdd(&count[color_bucket(d, i)], 1u);
+        atomicMax(&colors, d.color[i] + 1);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) d.ctr->colors = colors;
+    color_offsets(d, count);
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < d.n; i += blockDim.x) {
+        if (d.motion[i] != kDynamic) continue;
+        const uint32_t b = color_bucket(d, i);
+        place_in_order(d, i, d.ctr->color_off[b] + atomicAdd(&count[b], 1u));
     }
 }
 
 void launch_prepare(const Dev& d, const StepParams& sp, cudaStream_t s) {
-    k_prepare_bodies<<<blocks_for(d.n), kBlock, 0, s>>>(d, sp);
-    note_launch(blocks_for(d.n));
-    k_prepare_pairs<<<cap_blocks(d.cap_pair, 128), 128, 0, s>>>(d, sp);
-    note_launch(cap_blocks(d.cap_pair, 128));
+    const uint32_t grid = cap_blocks(std::max(d.cap_pair, d.n), 128);
+    k_prepare<<<grid, 128, 0, s>>>(d, sp);
+    note_launch(grid);
     if (d.nj) {
         k_prepare_joints<<<blocks_for(d.nj, 64), 64, 0, s>>>(d, sp);
         note_launch(blocks_for(d.nj, 64));
     }
-    launch_contact_jacobians(d, 0, sp.dt, s);
     prof_mark(s, "prepare");
 }
 
@@ -548,10 +606,15 @@ const void* color_kernel_ptr = reinterpret_cast<const void*>(&k_color);
 
 void launch_graph(const Dev& d, const StepParams& sp, cudaStream_t s, int coop_blocks) {
     uint32_t gb = cap_blocks(d.cap_pair > d.nj ? d.cap_pair : d.nj);
-    k_graph_degrees<<<gb, kBlock, 0, s>>>(d, sp);
-    note_launch(gb);
-    scan_u32(d.deg, d.inc_off, nullptr, d.n, nullptr, 0u, d.scan_tmp32, s);
-    scan_u32(d.jdeg, d.jinc_off, nullptr, d.n, nullptr, 0u, d.scan_tmp32, s);
+    const uint32_t db = cap_blocks(std::max({d.cap_pair, d.nj, d.cap_contact}));
+    k_graph_degrees<<<db, kBlock, 0, s>>>(d, sp);
+    note_launch(db);
+    // (Without joints the joint lists' offsets stay the zeros of the world's
+    // creation.)
+    if (d.nj)
+        scan_u32_pair(d.deg, d.inc_off, nullptr, d.jdeg, d.jinc_off, nullptr, nullptr, d.n, d.scan_tmp32, s);
+    else
+        scan_u32(d.deg, d.inc_off, nullptr, d.n, nullptr, 0u, d.scan_tmp32, s);
     k_graph_fill<<<gb, kBlock, 0, s>>>(d);
     note_launch(gb);
     k_graph_lists<<<blocks_for(d.n), kBlock, 0, s>>>(d);
@@ -559,27 +622,26 @@ void launch_graph(const Dev& d, const StepParams& sp, cudaStream_t s, int coop_b
     k_graph_roots<<<blocks_for(d.n), kBlock, 0, s>>>(d);
     note_launch(blocks_for(d.n));
     scan_u32(d.rcount, d.roff, nullptr, d.n, nullptr, 0u, d.scan_tmp32, s);
-    k_row_lists<<<blocks_for(d.n), kBlock, 0, s>>>(d);
-    note_launch(blocks_for(d.n));
-    k_graph_impact<<<cap_blocks(d.cap_pair), kBlock, 0, s>>>(d);
-    note_launch(cap_blocks(d.cap_pair));
-    k_graph_islands<<<blocks_for(d.n), kBlock, 0, s>>>(d);
-    note_launch(blocks_for(d.n));
-    prof_mark(s, "graph lists+islands");
-    k_neighbour_lists<<<blocks_for(d.n), kBlock, 0, s>>>(d);
-    note_launch(blocks_for(d.n));
+    const uint32_t rb = cap_blocks(std::max(d.cap_pair, d.n));
+    k_graph_rows<<<rb, kBlock, 0, s>>>(d);
+    note_launch(rb);
+    prof_mark(s, "graph lists");
     void* args[] = {const_cast<Dev*>(&d)};
     cudaLaunchCooperativeKernel(color_kernel_ptr, dim3(coop_blocks), dim3(kColorThreads), args, 0, s);
     note_launch(coop_blocks);
     prof_mark(s, "colour fixpoint");
-    k_color_count<<<blocks_for(d.n), kBlock, 0, s>>>(d);
-    note_launch(blocks_for(d.n));
-    static_assert(kPer * 1024 >= kBuckets, "bucket scan is one block");
-    k_color_offsets<<<1, 1024, 0, s>>>(d);
-    note_launch(1);
-    k_color_scatter<<<blocks_for(d.n), kBlock, 0, s>>>(d);
-    note_launch(blocks_for(d.n));
-    prof_mark(s, "colour buckets");
+    if (d.n <= kOneBlockOrder) {
+        k_color_order<<<1, 1024, 0, s>>>(d);
+        note_launch(1);
+    } else {
+        k_color_count<<<blocks_for(d.n), kBlock, 0, s>>>(d);
+        note_launch(blocks_for(d.n));
+        k_color_offsets<<<1, 1024, 0, s>>>(d);
+        note_launch(1);
+        k_color_scatter<<<blocks_for(d.n), kBlock, 0, s>>>(d);
+        note_launch(blocks_for(d.n));
+    }
+    prof_mark(s, "islands+colour order");
 }
 
 }  // namespace pmb

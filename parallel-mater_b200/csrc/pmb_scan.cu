@@ -66,9 +66,24 @@ __device__ __forceinline__ void store_items(T* out, uint32_t first, uint32_t cou
     }
 }
 
+// One scan of a launch (blockIdx.y picks it; scans of one length can share
+// their launches).
+template <class T> struct ScanJob {
+    const T* in;
+    T* out;
+    T* total;  // may be null
+    T* tiles;  // tile totals (long scans)
+};
+template <class T> struct ScanJobs {
+    ScanJob<T> job[2];
+};
+
 template <class T>
 __global__ void __launch_bounds__(kScanBlockThreads)
-    k_scan_block(const T* in, T* out, const uint32_t* count_ptr, uint32_t capacity, T* total, uint32_t total_cap) {
+    k_scan_block(ScanJobs<T> jobs, const uint32_t* count_ptr, uint32_t capacity, uint32_t total_cap) {
+    const T* in = jobs.job[blockIdx.y].in;
+    T* out = jobs.job[blockIdx.y].out;
+    T* total = jobs.job[blockIdx.y].total;
     const uint32_t count = count_ptr ? min(*count_ptr, capacity) : capacity;
     __shared__ T chunk;
     T carry = 0;
@@ -87,7 +102,9 @@ __global__ void __launch_bounds__(kScanBlockThreads)
 }
 
 template <class T>
-__global__ void k_tile_sums(const T* in, const uint32_t* count_ptr, uint32_t capacity, T* tile_sums) {
+__global__ void k_tile_sums(ScanJobs<T> jobs, const uint32_t* count_ptr, uint32_t capacity) {
+    const T* in = jobs.job[blockIdx.y].in;
+    T* tile_sums = jobs.job[blockIdx.y].tiles;
     const uint32_t count = count_ptr ? min(*count_ptr, capacity) : capacity;
     const uint32_t base = blockIdx.x * kScanTile;
     if (base >= count) return;  // totals past the end are never read
@@ -99,8 +116,11 @@ __global__ void k_tile_sums(const T* in, const uint32_t* count_ptr, uint32_t cap
 }
 
 template <class T>
-__global__ void k_scan_apply(const T* in, T* out, const uint32_t* count_ptr, uint32_t capacity, const T* tile_sums,
-                             T* total, uint32_t total_cap) {
+__global__ void k_scan_apply(ScanJobs<T> jobs, const uint32_t* count_ptr, uint32_t capacity, uint32_t total_cap) {
+    const T* in = jobs.job[blockIdx.y].in;
+    T* out = jobs.job[blockIdx.y].out;
+    T* total = jobs.job[blockIdx.y].total;
+    const T* tile_sums = jobs.job[blockIdx.y].tiles;
     const uint32_t count = count_ptr ? min(*count_ptr, capacity) : capacity;
     const uint32_t base = blockIdx.x * kScanTile;
     if (base >= count && !(blockIdx.x == 0 && count == 0)) return;
@@ -124,28 +144,35 @@ __global__ void k_scan_apply(const T* in, T* out, const uint32_t* count_ptr, uin
 // out holds capacity + 1 entries; out[count] receives the total and, when
 // `total` is non-null, *total the total or `total_cap` if that is less.
 template <class T>
-static void scan_impl(const T* in, T* out, const uint32_t* count_ptr, uint32_t capacity, T* total, uint32_t total_cap,
-                      T* tmp, cudaStream_t s) {
+static void scan_impl(const ScanJobs<T>& jobs, uint32_t njobs, const uint32_t* count_ptr, uint32_t capacity,
+                      uint32_t total_cap, cudaStream_t s) {
     if (capacity <= kScanBlockMost) {
-        k_scan_block<T><<<1, kScanBlockThreads, 0, s>>>(in, out, count_ptr, capacity, total, total_cap);
-        note_launch(1);
+        k_scan_block<T><<<dim3(1, njobs), kScanBlockThreads, 0, s>>>(jobs, count_ptr, capacity, total_cap);
+        note_launch(njobs);
         return;
     }
     const uint32_t tiles = (capacity + kScanTile - 1) / kScanTile;
-    k_tile_sums<T><<<tiles, kScanThreads, 0, s>>>(in, count_ptr, capacity, tmp);
-    note_launch(tiles);
-    k_scan_apply<T><<<tiles, kScanThreads, 0, s>>>(in, out, count_ptr, capacity, tmp, total, total_cap);
-    note_launch(tiles);
+    k_tile_sums<T><<<dim3(tiles, njobs), kScanThreads, 0, s>>>(jobs, count_ptr, capacity);
+    note_launch(tiles * njobs);
+    k_scan_apply<T><<<dim3(tiles, njobs), kScanThreads, 0, s>>>(jobs, count_ptr, capacity, total_cap);
+    note_launch(tiles * njobs);
 }
 
 void scan_u32(const uint32_t* in, uint32_t* out, const uint32_t* count_ptr, uint32_t capacity, uint32_t* total,
               uint32_t total_cap, uint32_t* tmp, cudaStream_t s) {
-    scan_impl<uint32_t>(in, out, count_ptr, capacity, total, total_cap, tmp, s);
+    scan_impl<uint32_t>({{{in, out, total, tmp}, {}}}, 1, count_ptr, capacity, total_cap, s);
+}
+
+void scan_u32_pair(const uint32_t* in0, uint32_t* out0, uint32_t* total0, const uint32_t* in1, uint32_t* out1,
+                   uint32_t* total1, const uint32_t* count_ptr, uint32_t capacity, uint32_t* tmp, cudaStream_t s) {
+    const uint32_t tiles = (capacity + kScanTile - 1) / kScanTile;
+    scan_impl<uint32_t>({{{in0, out0, total0, tmp}, {in1, out1, total1, tmp + tiles}}}, 2, count_ptr, capacity,
+                        0xffffffffu, s);
 }
 
 void scan_u64(const uint64_t* in, uint64_t* out, const uint32_t* count_ptr, uint32_t capacity, uint64_t* tmp,
               cudaStream_t s) {
-    scan_impl<uint64_t>(in, out, count_ptr, capacity, nullptr, 0u, tmp, s);
+    scan_impl<uint64_t>({{{in, out, nullptr, tmp}, {}}}, 1, count_ptr, capacity, 0u, s);
 }
 
 }  // namespace pmb

@@ -10,39 +10,54 @@
 // last-iteration work (accumulated impulses, re-anchoring sliding contacts) is
 // applied after the loop from the final duals and the stick flag each dual
 // pass stores, which is the same arithmetic on the same values.
+#include <algorithm>
+
 #include "pmb_solve_common.cuh"
 
 namespace pmb {
 
-// Each contact's phase record (d.c_row); its friction and penalty growth
-// factor come from the bodies' materials and masses. The velocity phase also
-// forms the force offsets (the row forces are the projected trial forces less
-// them): the normal impulse and the accumulated friction of the position
-// phase, both fixed by then (k_contact_finalize), over dt; its errors are
-// filled in by k_impact_constraints.
-__global__ void k_contact_jacobians(Dev d, uint32_t phase, float dt) {
-    if (phase != 0 && d.ctr->impact == 0) return;
+// The velocity phase's rows (geometry_constraints_solve.slang:238-330, after
+// k_impact_bodies has reset the targets): each contact's phase record with
+// its errors, its force offsets (the row forces are the projected trial
+// forces less them) -- the normal impulse and the accumulated friction of the
+// position phase, both fixed by then, over dt -- and the joints' rows.
+__global__ void k_impact_rows(Dev d, float dt, const float4* ov, const float4* ow) {
+    if (d.ctr->impact == 0) return;
+    for (uint32_t j = grid_stride_begin(); j < d.nj; j += grid_stride()) {
+        const JointState st = d.jstate[j];
+        if (st.count == 0 || !st.enabled) continue;
+        const uint32_t a = st.dense_a, b = st.dense_b;
+        if (d.impact[a] == 0 && d.impact[b] == 0) continue;
+        BodyView A = load_body(d, a), B = load_body(d, b);
+        Blk scratch;
+        visit_joint(d.joints[j], d.jrows + size_t(j) * 18, A, B, v3(d.x[a]), q4(d.q[a]), v3(d.x[b]), q4(d.q[b]),
+                    d.p0[a], d.p0[b], dt, &scratch, true, kVisitImpact, nullptr);
+    }
     const uint32_t n_con = d.ctr->n_contacts;
     for (uint32_t c = grid_stride_begin(); c < n_con; c += grid_stride()) {
         const uint2 ab = d.c_bodies[c];
         const uint32_t a = ab.x, b = ab.y;
         V6 ja[3], jb[3];
-        contact_jacobians(v3(d.c_n[c]), v3(d.c_p[c]), v3(d.c_aa[c]), v3(d.c_ab[c]), v3(d.tx[a]), q4(d.tq[a]),
-                          v3(d.tx[b]), q4(d.tq[b]), ja, jb);
-        const float friction = sqrtf(d.p1[a].x * d.p1[b].x);
-        const float beta = (1.0f / (fmx(d.p0[a].x + d.p0[b].x, 1.0e-6f) * dt * dt)) * 100.0f;
-        store_row32(d, c, ja, jb, friction, beta, d.c_e[c]);
-        if (phase != 0) {
-            V3 t0, t1;
-            basis(v3(d.c_n[c]), t0, t1);
-            const V3 af = v3(d.c_accf[c]);
-            d.c_foff[c] = make_float4(d.c_lam[c].w / dt, dot(af, t0) / dt, dot(af, t1) / dt, 0.0f);
+        float friction, beta;
+        contact_phase_row(d, c, a, b, dt, ja, jb, friction, beta);
+        float4 e = d.c_e[c];
+        if (d.impact[a] != 0 || d.impact[b] != 0) {
+            const V6 va = jac(mul(v3(ov[a]), dt), mul(v3(ow[a]), dt));
+            const V6 vb = jac(mul(v3(ov[b]), dt), mul(v3(ow[b]), dt));
+            const float gap = e.x, speed = e.w;
+            const bool cached = d.c_aa[c].w != 0.0f;
+            const float rest = !cached && speed < -1.0f ? fmn(d.p1[a].y, d.p1[b].y) : 0.0f;
+            e.x = dot6(ja[0], va) + dot6(jb[0], vb) - gap - rest * speed * dt;
+            e.y = dot6(ja[1], va) + dot6(jb[1], vb);
+            e.z = dot6(ja[2], va) + dot6(jb[2], vb);
+            d.c_e[c] = e;
         }
+        store_row32(d, c, ja, jb, friction, beta, e);
+        V3 t0, t1;
+        basis(v3(d.c_n[c]), t0, t1);
+        const V3 af = v3(d.c_accf[c]);
+        d.c_foff[c] = make_float4(d.c_lam[c].w / dt, dot(af, t0) / dt, dot(af, t1) / dt, 0.0f);
     }
-}
-void launch_contact_jacobians(const Dev& d, uint32_t phase, float dt, cudaStream_t s) {
-    k_contact_jacobians<<<cap_blocks(d.cap_contact), kBlock, 0, s>>>(d, phase, dt);
-    note_launch(cap_blocks(d.cap_contact));
 }
 
 // ------------------------------------------------------------ staged solve
@@ -705,8 +720,7 @@ const SolveVariant& solve_variant(uint32_t v) {
 
 // Last-iteration contact work (geometry_constraints_solve.slang:533-561),
 // one thread per contact point.
-__global__ void k_contact_finalize(Dev d, StepParams sp, uint32_t phase) {
-    if (phase != 0 && d.ctr->impact == 0) return;
+__device__ __forceinline__ void contact_finalize(const Dev& d, const StepParams& sp, uint32_t phase) {
     const float dt = sp.dt;
     const uint32_t n_con = d.ctr->n_contacts;
     for (uint32_t c = grid_stride_begin(); c < n_con; c += grid_stride()) {
@@ -745,7 +759,7 @@ __global__ void k_contact_finalize(Dev d, StepParams sp, uint32_t phase) {
 // free_mean (geometry_constraints_solve.slang:617-675): anchored flag per
 // island (any member touching a non-dynamic body), then the mass-weighted mean
 // of unanchored islands, summed serially in body order from the root.
-__global__ void k_free_anchor(Dev d, uint32_t phase) {
+__device__ __forceinline__ void free_anchor(const Dev& d) {
     const uint32_t n_act = d.ctr->n_act;
     for (uint32_t i = grid_stride_begin(); i < d.n; i += grid_stride()) d.mean[i] = make_float4(0, 0, 0, 0);
     for (uint32_t i = grid_stride_begin(); i < n_act; i += grid_stride()) {
@@ -761,6 +775,13 @@ __global__ void k_free_anchor(Dev d, uint32_t phase) {
         if (da && !db) d.anchored[d.parent[st.dense_a]] = 1;
         if (db && !da) d.anchored[d.parent[st.dense_b]] = 1;
     }
+}
+
+// Both need only the solved displacements.
+__global__ void k_finish_contacts(Dev d, StepParams sp, uint32_t phase) {
+    if (phase != 0 && d.ctr->impact == 0) return;
+    contact_finalize(d, sp, phase);
+    free_anchor(d);
 }
 
 // One warp per island root: the members, found 32 indices at a time between
@@ -802,27 +823,21 @@ __global__ void k_free_mean(Dev d, uint32_t phase) {
     }
 }
 
-__global__ void k_free_subtract(Dev d, uint32_t phase) {
-    for (uint32_t i = grid_stride_begin(); i < d.n; i += grid_stride()) {
-        if (d.motion[i] != kDynamic || (phase != 0 && d.impact[i] == 0)) continue;
-        const float4 m = d.mean[d.parent[i]];
-        float4 l = d.dx[2 * i];
-        l.x -= m.x;
-        l.y -= m.y;
-        l.z -= m.z;
-        d.dx[2 * i] = l;
-    }
-}
-
-// apply_states (geometry_constraints_solve.slang:699-733) into the output
-// state arrays (v: solved state; t: the AVBD target stays untouched).
+// The free islands' means taken off, then apply_states
+// (geometry_constraints_solve.slang:676-733) into the output state arrays (v: solved state; t: the AVBD target stays untouched).
 __global__ void k_apply(Dev d, StepParams sp, uint32_t phase, float4* ox, float4* oq, float4* ov, float4* ow) {
     if (phase != 0 && d.ctr->impact == 0) return;
     const float dt = sp.dt;
     for (uint32_t i = grid_stride_begin(); i < d.n; i += grid_stride()) {
         if (d.motion[i] != kDynamic) continue;
         if (phase != 0 && d.impact[i] == 0) continue;
-        const float4 l = d.dx[2 * i], a = d.dx[2 * i + 1];
+        const float4 m = d.mean[d.parent[i]];
+        float4 l = d.dx[2 * i];
+        const float4 a = d.dx[2 * i + 1];
+        l.x -= m.x;
+        l.y -= m.y;
+        l.z -= m.z;
+        d.dx[2 * i] = l;
         const V3 lin = v3(l), rot = v3(a);
         V3 x = v3(d.tx[i]), v = v3(d.tv[i]), w = v3(d.tw[i]);
         Q4 q = q4(d.tq[i]);
@@ -908,46 +923,12 @@ __global__ void k_impact_bodies(Dev d, const float4* ox, const float4* oq, const
         }
     }
 }
-__global__ void k_impact_constraints(Dev d, StepParams sp, const float4* ov, const float4* ow) {
-    if (d.ctr->impact == 0) return;
-    const float dt = sp.dt;
-    for (uint32_t j = grid_stride_begin(); j < d.nj; j += grid_stride()) {
-        const JointState st = d.jstate[j];
-        if (st.count == 0 || !st.enabled) continue;
-        const uint32_t a = st.dense_a, b = st.dense_b;
-        if (d.impact[a] == 0 && d.impact[b] == 0) continue;
-        BodyView A = load_body(d, a), B = load_body(d, b);
-        Blk scratch;
-        visit_joint(d.joints[j], d.jrows + size_t(j) * 18, A, B, v3(d.x[a]), q4(d.q[a]), v3(d.x[b]), q4(d.q[b]),
-                    d.p0[a], d.p0[b], dt, &scratch, true, kVisitImpact, nullptr);
-    }
-    const uint32_t n_act = d.ctr->n_act;
-    for (uint32_t i = grid_stride_begin(); i < n_act; i += grid_stride()) {
-        const uint32_t a = d.act_a[i], b = d.act_b[i];
-        if (d.impact[a] == 0 && d.impact[b] == 0) continue;
-        const V6 va = jac(mul(v3(ov[a]), dt), mul(v3(ow[a]), dt));
-        const V6 vb = jac(mul(v3(ov[b]), dt), mul(v3(ow[b]), dt));
-        const float rest_ab = fmn(d.p1[a].y, d.p1[b].y);
-        for (uint32_t q = d.act_off[i]; q < d.act_off[i] + d.act_cnt[i]; ++q) {
-            float4 e = d.c_e[q];
-            const float gap = e.x;
-            const ContactRow cr = load_row32(d, q);  // recomputed from the reset targets
-            const bool cached = d.c_aa[q].w != 0.0f;
-            const float speed = e.w;
-            const float rest = !cached && speed < -1.0f ? rest_ab : 0.0f;
-            e.x = dot6(cr.ja(0), va) + dot6(cr.jb(0), vb) - gap - rest * speed * dt;
-            e.y = dot6(cr.ja(1), va) + dot6(cr.jb(1), vb);
-            e.z = dot6(cr.ja(2), va) + dot6(cr.jb(2), vb);
-            d.c_e[q] = e;
-            // The record's errors (its last float4: growth factor, errors).
-            d.c_row[size_t(q) * 8 + 7] = make_float4(cr.beta, e.x, e.y, e.z);
-        }
-    }
-}
-
 // pm_clamp_rigid_speeds (geometry.slang:3086-3100), then commit the solved
-// states as the next tick's current states.
-__global__ void k_clamp_commit(Dev d, const float4* ox, const float4* oq, const float4* ov, const float4* ow) {
+// states as the next tick's current states; and pm_save_rigid_contact_cache
+// (geometry.slang:3011-3070) into the next tick's cache buffers, keyed by
+// pair code (already sorted).
+__global__ void k_commit(Dev d, StepParams sp, const float4* ox, const float4* oq, const float4* ov,
+                         const float4* ow) {
     for (uint32_t i = grid_stride_begin(); i < d.n; i += grid_stride()) {
         V3 v = v3(ov[i]), w = v3(ow[i]);
         if (d.motion[i] == kDynamic) {
@@ -960,11 +941,6 @@ __global__ void k_clamp_commit(Dev d, const float4* ox, const float4* oq, const 
         d.v[i] = f4(v);
         d.w[i] = f4(w);
     }
-}
-
-// pm_save_rigid_contact_cache (geometry.slang:3011-3070) into the next tick's
-// cache buffers, keyed by pair code (already sorted).
-__global__ void k_cache_save(Dev d, StepParams sp) {
     const uint32_t n_act = d.ctr->n_act;
     if (grid_stride_begin() == 0) {
         *d.out_n_pairs = n_act;
@@ -972,8 +948,8 @@ __global__ void k_cache_save(Dev d, StepParams sp) {
     }
     for (uint32_t i = grid_stride_begin(); i < n_act; i += grid_stride()) {
         const uint32_t a = d.act_a[i];
-        const V3 xa = v3(d.x[a]);
-        const Q4 qa = q4(d.q[a]);
+        const V3 xa = v3(ox[a]);
+        const Q4 qa = q4(oq[a]);
         const uint32_t off = d.act_off[i], np = d.act_cnt[i];
         d.out_code[i] = d.act_code[i];
         d.out_off[i] = off;
@@ -1025,15 +1001,15 @@ void launch_solve_all(const Dev& d, const StepParams& sp, cudaStream_t s, int co
     const SolveVariant& sv = solve_variant(d.solve_variant);
     const int coop = coop_blocks;
     const int feat = solve_features(d);
-    const uint32_t pb = cap_blocks(d.cap_pair > d.nj ? d.cap_pair : d.nj);
+    const uint32_t pb = cap_blocks(std::max(d.cap_contact, d.nj)), nb = cap_blocks(std::max(d.cap_pair, d.n));
+    const uint32_t fb = cap_blocks(std::max({d.cap_contact, d.cap_pair, d.n, d.nj}));
     for (uint32_t phase = 0; phase < (sp.realtime ? 1u : 2u); ++phase) {
         if (phase != 0) {
             k_impact_setup<<<cap_blocks(d.cap_pair), kBlock, 0, s>>>(d, sp, o.ox, o.oq, o.ov, o.ow);
             note_launch(cap_blocks(d.cap_pair));
             k_impact_bodies<<<blocks_for(d.n), kBlock, 0, s>>>(d, o.ox, o.oq, o.ov, o.ow);
             note_launch(blocks_for(d.n));
-            launch_contact_jacobians(d, 1, sp.dt, s);
-            k_impact_constraints<<<pb, kBlock, 0, s>>>(d, sp, o.ov, o.ow);
+            k_impact_rows<<<pb, kBlock, 0, s>>>(d, sp.dt, o.ov, o.ow);
             note_launch(pb);
             prof_mark(s, "impact setup");
         }
@@ -1049,14 +1025,10 @@ void launch_solve_all(const Dev& d, const StepParams& sp, cudaStream_t s, int co
         note_launch(coop);
         solve_timer_end(s);
         prof_mark(s, phase ? "solve phase 1" : "solve phase 0");
-        k_contact_finalize<<<cap_blocks(d.cap_contact), kBlock, 0, s>>>(d, sp, phase);
-        note_launch(cap_blocks(d.cap_contact));
-        k_free_anchor<<<cap_blocks(d.cap_pair > d.n ? d.cap_pair : d.n), kBlock, 0, s>>>(d, phase);
-        note_launch(cap_blocks(d.cap_pair > d.n ? d.cap_pair : d.n));
+        k_finish_contacts<<<fb, kBlock, 0, s>>>(d, sp, phase);
+        note_launch(fb);
         k_free_mean<<<std::min<uint32_t>(blocks_for(32u * d.n, 256), 148u * 8u), 256, 0, s>>>(d, phase);
         note_launch(std::min<uint32_t>(blocks_for(32u * d.n, 256), 148u * 8u));
-        k_free_subtract<<<blocks_for(d.n), kBlock, 0, s>>>(d, phase);
-        note_launch(blocks_for(d.n));
         k_apply<<<blocks_for(d.n), kBlock, 0, s>>>(d, sp, phase, o.ox, o.oq, o.ov, o.ow);
         note_launch(blocks_for(d.n));
         if (phase == 0 && d.n_hinge_segs) {
@@ -1066,10 +1038,8 @@ void launch_solve_all(const Dev& d, const StepParams& sp, cudaStream_t s, int co
         prof_mark(s, phase ? "finish phase 1" : "finish phase 0");
     }
     set_phase(kPhCommit);
-    k_clamp_commit<<<blocks_for(d.n), kBlock, 0, s>>>(d, o.ox, o.oq, o.ov, o.ow);
-    note_launch(blocks_for(d.n));
-    k_cache_save<<<cap_blocks(d.cap_pair), kBlock, 0, s>>>(d, sp);
-    note_launch(cap_blocks(d.cap_pair));
+    k_commit<<<nb, kBlock, 0, s>>>(d, sp, o.ox, o.oq, o.ov, o.ow);
+    note_launch(nb);
     if (sp.collect_events && d.event_capacity) {
         k_contact_events<<<cap_blocks(d.event_capacity), kBlock, 0, s>>>(d);
         note_launch(cap_blocks(d.event_capacity));

@@ -19,8 +19,7 @@ __device__ __forceinline__ Lite load_lite(const Dev& d, uint32_t i) {
 
 // Contact jacobians (geometry_constraints.slang:508-532). They depend only on
 // the contact geometry and the AVBD target poses, both fixed during a solve
-// phase, so they are evaluated once per phase (k_contact_jacobians) and
-// stored in the contact's phase record (d.c_row).
+// phase, so they are evaluated once per phase and stored in the contact's phase record (d.c_row).
 __device__ __forceinline__ void contact_jacobians(V3 n, V3 pt, V3 anc_a, V3 anc_b, V3 xa, Q4 qa, V3 xb, Q4 qb,
                                                   V6 ja[3], V6 jb[3]) {
     V3 t0, t1;
@@ -89,6 +88,15 @@ __device__ __forceinline__ void store_row32(const Dev& d, uint32_t c, const V6 j
     float4* p = d.c_row + size_t(c) * 8;
 #pragma unroll
     for (int k = 0; k < 8; ++k) p[k] = make_float4(f[4 * k], f[4 * k + 1], f[4 * k + 2], f[4 * k + 3]);
+}
+// Contact c's values of a phase: its jacobians at the phase's target poses,
+// its friction and penalty growth factor (its bodies' materials and masses).
+__device__ __forceinline__ void contact_phase_row(const Dev& d, uint32_t c, uint32_t a, uint32_t b, float dt, V6 ja[3],
+                                                  V6 jb[3], float& friction, float& beta) {
+    contact_jacobians(v3(d.c_n[c]), v3(d.c_p[c]), v3(d.c_aa[c]), v3(d.c_ab[c]), v3(d.tx[a]), q4(d.tq[a]), v3(d.tx[b]),
+                      q4(d.tq[b]), ja, jb);
+    friction = sqrtf(d.p1[a].x * d.p1[b].x);
+    beta = (1.0f / (fmx(d.p0[a].x + d.p0[b].x, 1.0e-6f) * dt * dt)) * 100.0f;
 }
 // The rows' errors at the bodies' displacements: e + J_a . dx_a + J_b . dx_b.
 __device__ __forceinline__ void contact_errors(const ContactRow& r, const Lite& A, const Lite& B, float err[3]) {

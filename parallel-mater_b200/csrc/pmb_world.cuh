@@ -366,6 +366,9 @@ void launch_body_constants(const Dev& d, const float4* lo, const float4* hi, con
 void launch_finish(const Dev& d, const StepParams& sp, cudaStream_t s);
 void scan_u32(const uint32_t* in, uint32_t* out, const uint32_t* count_ptr, uint32_t capacity, uint32_t* total,
               uint32_t total_cap, uint32_t* tmp, cudaStream_t s);
+// Two scans of the same length in the launches of one (tmp for both).
+void scan_u32_pair(const uint32_t* in0, uint32_t* out0, uint32_t* total0, const uint32_t* in1, uint32_t* out1,
+                   uint32_t* total1, const uint32_t* count_ptr, uint32_t capacity, uint32_t* tmp, cudaStream_t s);
 void scan_u64(const uint64_t* in, uint64_t* out, const uint32_t* count_ptr, uint32_t capacity, uint64_t* tmp,
               cudaStream_t s);
 void release_bvh_scratch(int device);  // gives back the mesh BVH builds' kept scratch
@@ -418,7 +421,6 @@ inline int solve_features(const Dev& d) { return (d.nj ? kFeatJoints : 0) | (d.s
 SolveVariant solve_group_variant_512();
 SolveVariant solve_group_variant_384();
 SolveVariant solve_group_variant_256();
-void launch_contact_jacobians(const Dev& d, uint32_t phase, float dt, cudaStream_t s);
 // Sparse per-body record writes staged in io_index / io_rec (kind 0: inputs,
 // 1: kinematic targets, 2: states), and AoS state packing into `dst`.
 void launch_scatter_records(const Dev& d, uint32_t kind, uint32_t count, cudaStream_t s);
