@@ -45,6 +45,7 @@ __device__ __forceinline__ int4 cell_of(float4 lo, float4 hi, float hs) {
 // operation order: reach = |centre| + radius + margin + 1e-5 and
 // correction = min(0.5, 0.25 * max(0, min extent)) for dynamic bodies.
 __global__ void k_body_constants(Dev d, const float4* mesh_lo, const float4* mesh_hi, const float4* mesh_sphere) {
+    tick_begin();
     for (uint32_t i = grid_stride_begin(); i < d.n; i += grid_stride()) {
         uint32_t m = d.mesh[i];
         V3 lo = v3(mesh_lo[m]), hi = v3(mesh_hi[m]);
@@ -64,11 +65,11 @@ __global__ void k_body_constants(Dev d, const float4* mesh_lo, const float4* mes
     }
 }
 void launch_body_constants(const Dev& d, const float4* lo, const float4* hi, const float4* sph, cudaStream_t s) {
-    k_body_constants<<<blocks_for(d.n), kBlock, 0, s>>>(d, lo, hi, sph);
-    note_launch(blocks_for(d.n));
+    launch(k_body_constants, blocks_for(d.n), kBlock, s, d, lo, hi, sph);
 }
 
 __global__ void k_integrate(Dev d, StepParams sp, float4* ox, float4* oq, float4* ov, float4* ow) {
+    tick_begin();
     const float dt = sp.dt;
     const V3 g{sp.gx, sp.gy, sp.gz};
     // The grid's counts and cursors of this tick (a memset each otherwise).
@@ -166,6 +167,7 @@ __global__ void k_integrate(Dev d, StepParams sp, float4* ox, float4* oq, float4
 // consumed and cleared by the next predictor, as pm_clear_rigid_inputs
 // (src/slang/geometry.slang:2877-2886) does at the end of the reference tick.
 __global__ void k_scatter_records(Dev d, uint32_t kind, uint32_t count) {
+    tick_begin();
     for (uint32_t k = grid_stride_begin(); k < count; k += grid_stride()) {
         const uint32_t b = d.io_index[k];
         if (b >= d.n) continue;
@@ -192,13 +194,13 @@ __global__ void k_scatter_records(Dev d, uint32_t kind, uint32_t count) {
 }
 void launch_scatter_records(const Dev& d, uint32_t kind, uint32_t count, cudaStream_t s) {
     if (count == 0) return;
-    k_scatter_records<<<blocks_for(count), kBlock, 0, s>>>(d, kind, count);
-    note_launch(blocks_for(count));
+    launch(k_scatter_records, blocks_for(count), kBlock, s, d, kind, count);
 }
 
 // States [first, first + count) as packed 13-float records (position,
 // orientation xyzw, linear and angular velocity) at dst.
 __global__ void k_pack_states(Dev d, uint32_t first, uint32_t count, float* dst) {
+    tick_begin();
     for (uint32_t k = grid_stride_begin(); k < count; k += grid_stride()) {
         const uint32_t b = first + k;
         const float4 x = d.x[b], q = d.q[b], v = d.v[b], w = d.w[b];
@@ -212,6 +214,7 @@ __global__ void k_pack_states(Dev d, uint32_t first, uint32_t count, float* dst)
 // The inverse for every body: x, q, v, w exactly as given (no
 // renormalisation, unlike the record writes).
 __global__ void k_unpack_states(Dev d, uint32_t count, const float* src) {
+    tick_begin();
     for (uint32_t b = grid_stride_begin(); b < count; b += grid_stride()) {
         const float* o = src + 13 * size_t(b);
         d.x[b] = make_float4(o[0], o[1], o[2], 0.0f);
@@ -222,22 +225,20 @@ __global__ void k_unpack_states(Dev d, uint32_t count, const float* src) {
 }
 void launch_unpack_states(const Dev& d, uint32_t count, const float* src, cudaStream_t s) {
     if (count == 0) return;
-    k_unpack_states<<<blocks_for(count), kBlock, 0, s>>>(d, count, src);
-    note_launch(blocks_for(count));
+    launch(k_unpack_states, blocks_for(count), kBlock, s, d, count, src);
 }
 void launch_pack_states(const Dev& d, uint32_t first, uint32_t count, float* dst, cudaStream_t s) {
     if (count == 0) return;
-    k_pack_states<<<blocks_for(count), kBlock, 0, s>>>(d, first, count, dst);
-    note_launch(blocks_for(count));
+    launch(k_pack_states, blocks_for(count), kBlock, s, d, first, count, dst);
 }
 
 void launch_integrate(const Dev& d, const StepParams& sp, cudaStream_t s, const SolveBuffers& o) {
-    k_integrate<<<blocks_for(d.n), kBlock, 0, s>>>(d, sp, o.ox, o.oq, o.ov, o.ow);
-    note_launch(blocks_for(d.n));
+    launch(k_integrate, blocks_for(d.n), kBlock, s, d, sp, o.ox, o.oq, o.ov, o.ow);
     prof_mark(s, "integrate+proxy");
 }
 
 __global__ void k_grid_count(Dev d) {
+    tick_begin();
     for (uint32_t i = grid_stride_begin(); i < d.n; i += grid_stride()) {
         if (d.is_large[i] != 0) continue;
         const float h = batched(d) ? d.scene_hs[d.scene_of[i]] : d.ctr->hs;
@@ -248,6 +249,7 @@ __global__ void k_grid_count(Dev d) {
 }
 
 __global__ void k_grid_scatter(Dev d) {
+    tick_begin();
     for (uint32_t i = grid_stride_begin(); i < d.n; i += grid_stride()) {
         if (d.is_large[i] != 0) continue;
         int4 c = d.grid_cell[i];
@@ -261,6 +263,7 @@ __global__ void k_grid_scatter(Dev d) {
 // kOneBlockGrid buckets (half as many bodies), where three launches cost more.
 constexpr uint32_t kOneBlockGrid = 8192;
 __global__ void __launch_bounds__(1024) k_grid_build(Dev d) {
+    tick_begin();
     __shared__ uint32_t count[kOneBlockGrid];
     __shared__ uint32_t part[32];
     constexpr uint32_t kPer = kOneBlockGrid / 1024;
@@ -360,6 +363,7 @@ __device__ __forceinline__ uint32_t group_root(const volatile uint32_t* root, ui
 // result does not depend on the order the joints are taken in. Each loop is
 // bounded by the body count (a failed swap means another union progressed).
 __global__ void __launch_bounds__(1024) k_fixed_groups(Dev d) {
+    tick_begin();
     volatile uint32_t* root = d.fixed_root;
     for (uint32_t i = threadIdx.x; i < d.n; i += blockDim.x) root[i] = i;
     __syncthreads();
@@ -429,11 +433,13 @@ __device__ uint32_t visit_candidates(const Dev& d, uint32_t a, uint32_t gl, uint
 
 // Per-scene large-body lists (batched worlds): count, offsets, scatter.
 __global__ void k_scene_large_count(Dev d) {
+    tick_begin();
     const uint32_t nl = d.ctr->n_large;
     for (uint32_t k = grid_stride_begin(); k < nl; k += grid_stride())
         atomicAdd(&d.scene_large_count[d.scene_of[d.large_list[k]]], 1u);
 }
 __global__ void k_scene_large_scatter(Dev d) {
+    tick_begin();
     const uint32_t nl = d.ctr->n_large;
     for (uint32_t k = grid_stride_begin(); k < nl; k += grid_stride()) {
         const uint32_t b = d.large_list[k], s = d.scene_of[b];
@@ -444,6 +450,7 @@ __global__ void k_scene_large_scatter(Dev d) {
 // kQueryLanes lanes per query body; each lane's count is kept for the
 // write pass.
 __global__ void k_query_count(Dev d) {
+    tick_begin();
     const uint32_t gl = threadIdx.x % kQueryLanes;
     const uint32_t gmask = ((1u << kQueryLanes) - 1u) << (threadIdx.x & 31u & ~(kQueryLanes - 1u));
     const uint32_t groups = grid_stride() / kQueryLanes;
@@ -457,6 +464,7 @@ __global__ void k_query_count(Dev d) {
 }
 
 __global__ void k_query_write(Dev d) {
+    tick_begin();
     // n_cand is the total clamped to the capacity (by the scan).
     if (grid_stride_begin() == 0 && d.cand_off[d.n] > d.cap_cand) atomicOr(&d.ctr->status, kStCandidateOverflow);
     const uint32_t gl = threadIdx.x % kQueryLanes;
@@ -491,34 +499,26 @@ __global__ void k_query_write(Dev d) {
 
 void launch_broadphase(const Dev& d, cudaStream_t s) {
     if (d.n_scenes > 1) {
-        k_scene_large_count<<<blocks_for(d.n), kBlock, 0, s>>>(d);
-        note_launch(blocks_for(d.n));
+        launch(k_scene_large_count, blocks_for(d.n), kBlock, s, d);
         scan_u32(d.scene_large_count, d.scene_large_off, nullptr, d.n_scenes, nullptr, 0u, d.scan_tmp32, s);
-        k_scene_large_scatter<<<blocks_for(d.n), kBlock, 0, s>>>(d);
-        note_launch(blocks_for(d.n));
+        launch(k_scene_large_scatter, blocks_for(d.n), kBlock, s, d);
     }
     if (d.grid_size <= kOneBlockGrid) {
-        k_grid_build<<<1, 1024, 0, s>>>(d);
-        note_launch(1);
+        launch(k_grid_build, 1, 1024, s, d);
     } else {
-        k_grid_count<<<blocks_for(d.n), kBlock, 0, s>>>(d);
-        note_launch(blocks_for(d.n));
+        launch(k_grid_count, blocks_for(d.n), kBlock, s, d);
         scan_u32(d.bucket_count, d.bucket_off, nullptr, d.grid_size, nullptr, 0u, d.scan_tmp32, s);
-        k_grid_scatter<<<blocks_for(d.n), kBlock, 0, s>>>(d);
-        note_launch(blocks_for(d.n));
+        launch(k_grid_scatter, blocks_for(d.n), kBlock, s, d);
     }
     prof_mark(s, "grid build");
     set_phase(kPhCandidates);
     if (d.n_fixed) {
-        k_fixed_groups<<<1, 1024, 0, s>>>(d);
-        note_launch(1);
+        launch(k_fixed_groups, 1, 1024, s, d);
     }
-    k_query_count<<<blocks_for(kQueryLanes * d.n, 128), 128, 0, s>>>(d);
-    note_launch(blocks_for(kQueryLanes * d.n, 128));
+    launch(k_query_count, blocks_for(kQueryLanes * d.n, 128), 128, s, d);
     prof_mark(s, "query count");
     scan_u32(d.cand_count, d.cand_off, nullptr, d.n, &d.ctr->n_cand, d.cap_cand, d.scan_tmp32, s);
-    k_query_write<<<blocks_for(kQueryLanes * d.n, 128), 128, 0, s>>>(d);
-    note_launch(blocks_for(kQueryLanes * d.n, 128));
+    launch(k_query_write, blocks_for(kQueryLanes * d.n, 128), 128, s, d);
     prof_mark(s, "query write");
 }
 

@@ -158,6 +158,7 @@ StepParams params_from(const pmb_step_desc& s) {
 
 // Also the per-scene sums that the predictor and the large-body lists add to.
 __global__ void k_reset_counters(Dev d) {
+    tick_begin();
     uint32_t* w = reinterpret_cast<uint32_t*>(d.ctr);
     const uint32_t words = sizeof(Counters) / 4;
     for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) w[i] = 0;
@@ -200,8 +201,7 @@ void enqueue_step(pmb_world* w, const StepParams& sp) {
     w->ledger = LaunchLedger{};
     g_ledger = &w->ledger;
     set_phase(kPhBoundary);
-    k_reset_counters<<<1, 1024, 0, s>>>(d);
-    note_launch(1);
+    launch(k_reset_counters, 1, 1024, s, d);
     set_phase(kPhPredict);
     launch_integrate(d, sp, s, w->out);
     set_phase(kPhIndex);

@@ -742,6 +742,7 @@ __device__ void mesh_walk(const Dev& d, const PairSetup& p, uint32_t pair, bool 
 }
 
 __global__ void k_mesh_walk_count(Dev d) {
+    tick_begin();
     const uint32_t total = min(d.ctr->n_mesh, d.cap_mesh);
     for (uint32_t s = grid_stride_begin(); s < total; s += grid_stride()) {
         const PairSetup p = pair_setup(d, d.np_mesh[s]);
@@ -770,6 +771,7 @@ __global__ void k_mesh_walk_count(Dev d) {
 }
 
 __global__ void k_mesh_walk_write(Dev d) {
+    tick_begin();
     const uint32_t total = min(d.ctr->n_mesh, d.cap_mesh);
     for (uint32_t s = grid_stride_begin(); s < total; s += grid_stride()) {
         if (!d.mp_leaves[s]) continue;
@@ -787,6 +789,7 @@ __global__ void k_mesh_walk_write(Dev d) {
 // single range of an overflowed traversal has more and loops), one lane per
 // triangle-pair item.
 __global__ void __launch_bounds__(128, 4) k_mesh_items(Dev d, StepParams sp) {
+    tick_begin();
     const uint32_t leaves_total = min(d.ctr->n_mesh_leaves, d.cap_mesh_leaves);
     const uint32_t items_total = min(d.ctr->n_mesh_items, d.cap_mesh_items);
     const uint32_t lane = threadIdx.x & 31u;
@@ -869,6 +872,7 @@ __device__ __forceinline__ void mm_add_lanes(WarpMan& m, uint32_t lane, V3 p, V3
 // items, most without a contact, took 186 us for 64 concave scenes. A guided
 // pair's merge (rare) stays with lane 0.
 __global__ void k_mesh_merge(Dev d, StepParams sp) {
+    tick_begin();
     const uint32_t pairs = min(d.ctr->n_mesh, d.cap_mesh);
     const uint32_t total = min(d.ctr->n_mesh_items, d.cap_mesh_items);
     const uint32_t lane = threadIdx.x & 31u;
@@ -1018,6 +1022,7 @@ __device__ float4 hinge_frame_at(const Dev& d, uint32_t i, const float4* pos, co
 // static body, gives the frame; a fixed joint marks a fixed member; an axial
 // frame needs the body's only joint. One thread per body.
 __global__ void k_hinge_frames(Dev d) {
+    tick_begin();
     for (uint32_t i = grid_stride_begin(); i < d.n; i += grid_stride()) {
         float4 guide, guide_anchor;
         d.frame[i] = hinge_frame_at(d, i, d.tx, d.tq, &guide, &guide_anchor);
@@ -1032,28 +1037,23 @@ __global__ void k_hinge_frames(Dev d) {
 
 void launch_hinge_frames(const Dev& d, cudaStream_t s) {
     if (!d.nj) return;
-    k_hinge_frames<<<blocks_for(d.n), kBlock, 0, s>>>(d);
-    note_launch(blocks_for(d.n));
+    launch(k_hinge_frames, blocks_for(d.n), kBlock, s, d);
 }
 
 void launch_mesh_narrowphase(const Dev& d, const StepParams& sp, cudaStream_t s) {
     const uint32_t pairs_grid = cap_blocks(d.cap_mesh, 128);
-    k_mesh_walk_count<<<pairs_grid, 128, 0, s>>>(d);
-    note_launch(pairs_grid);
+    launch(k_mesh_walk_count, pairs_grid, 128, s, d);
     prof_mark(s, "mesh walk");
     scan_u32_pair(d.mp_leaves, d.mp_leaf_off, &d.ctr->n_mesh_leaves, d.mp_items, d.mp_item_off, &d.ctr->n_mesh_items,
                   &d.ctr->n_mesh, d.cap_mesh, d.scan_tmp32, s);
     prof_mark(s, "mesh scans");
-    k_mesh_walk_write<<<pairs_grid, 128, 0, s>>>(d);
-    note_launch(pairs_grid);
+    launch(k_mesh_walk_write, pairs_grid, 128, s, d);
     prof_mark(s, "mesh leaf pairs");
     const uint32_t items_grid = cap_blocks(32 * size_t(d.cap_mesh_leaves), 128);
-    k_mesh_items<<<items_grid, 128, 0, s>>>(d, sp);
-    note_launch(items_grid);
+    launch(k_mesh_items, items_grid, 128, s, d, sp);
     prof_mark(s, "mesh triangle pairs");
     const uint32_t merge_grid = cap_blocks(32 * size_t(d.cap_mesh), 128);
-    k_mesh_merge<<<merge_grid, 128, 0, s>>>(d, sp);
-    note_launch(merge_grid);
+    launch(k_mesh_merge, merge_grid, 128, s, d, sp);
 }
 
 }  // namespace pmb

@@ -2,7 +2,7 @@
 // Convex face narrowphase, manifold compaction and the persistent contact
 // cache.
 //
-// One thread per candidate pair runs the reference's convex face contact:
+// A candidate pair runs the reference's convex face contact:
 // SAT over every reference-face plane of both meshes (support = min over the
 // incident mesh's vertices), most anti-aligned incident face, Sutherland-
 // Hodgman clipping of each incident triangle coplanar with it against the
@@ -317,11 +317,24 @@ __device__ __forceinline__ void to_mesh_path(const Dev& d, uint32_t k) {
     d.np_mesh[slot] = k;
 }
 
+// A pair without a face manifold.
+__device__ __forceinline__ void declined(const Dev& d, uint32_t k, uint32_t a, uint32_t b) {
+    // Most declined pairs lie beyond the pair margin: their root bounds (the
+    // mesh path's first test) settle them here.
+    if (mesh_pair_bounds_overlap(d, a, b, false)) {
+        to_mesh_path(d, k);
+    } else {
+        d.np_count[k] = 0;
+        d.np_scan[k] = 0ull;
+    }
+}
+
 // Pass 1, one thread per candidate: pairs that are not both face-capable, and
 // guided pairs, go to the triangle-mesh path; unswept pairs separated by a
 // face plane get an empty manifold here; the rest go to the survivor list for
 // pass 2 with their separating-axis result. Light enough for full occupancy.
 __global__ void __launch_bounds__(256) k_narrow_sat(Dev d) {
+    tick_begin();
     const uint32_t total = d.ctr->n_cand;
     for (uint32_t k = grid_stride_begin(); k < total; k += grid_stride()) {
         const uint32_t a = d.cand_a[k], b = d.cand_b[k];
@@ -352,61 +365,470 @@ __global__ void __launch_bounds__(256) k_narrow_sat(Dev d) {
     }
 }
 
-// Pass 2, one thread per surviving candidate: the full face manifold
-// (swept variant first when the pair moved more than its margin).
+// ---- pass 2: the face manifold of a surviving candidate by 16 lanes
+//
+// In one thread a manifold is a serial chain of clipped vertices kept in
+// local memory: 12 planes x 2 triangles x 6 vertices and the contact merge
+// took 124 us however few the pairs. Here a lane holds a vertex of the polygon
+// being clipped: a plane's distances, intersections and the new vertices'
+// places (from two ballots) are formed side by side, and so are the support
+// planes, the incident face, the merge's comparisons and the collinear test.
+// Every value is the serial code's, from the same operands; what the serial
+// order decides -- the first of equal faces, the vertices' order, the first
+// near contact, the first collinear triple -- is decided by the lowest lane or
+// index. 16 lanes hold any clip of a box by a box (at most 15 vertices); a
+// polygon that outgrows them (meshes of up to 32 faces) sends its pair to the
+// serial code.
+constexpr int kClipLanes = 16;
+constexpr int kNarrowThreads = 128;
+struct ClipShared {
+    float4 poly[2][kClipLanes];
+    float4 man[8];
+};
+struct LaneGroup {
+    uint32_t mask;
+    int gl, base;
+    __device__ __forceinline__ uint32_t ballot(bool p) const { return (__ballot_sync(mask, p) >> base) & 0xffffu; }
+    __device__ __forceinline__ float from(float v, int lane) const { return __shfl_sync(mask, v, base + lane); }
+    __device__ __forceinline__ uint32_t from(uint32_t v, int lane) const { return __shfl_sync(mask, v, base + lane); }
+};
+
+// The first face of the largest separation, as face_sat. Pairs (value, order)
+// reduce to the largest value of the lowest order.
+__device__ __forceinline__ FaceSat face_sat_lanes(const LaneGroup& g, const Pose& bs, const MeshRef& bm,
+                                                  const Pose& cs, const MeshRef& cm) {
+    float best = -kFltMax;
+    uint32_t order = 0xffffffffu;
+    for (uint32_t side = 0; side < 2; ++side) {
+        const MeshRef& rm = side == 0 ? cm : bm;
+        const Pose& rs = side == 0 ? cs : bs;
+        const MeshRef& im = side == 0 ? bm : cm;
+        const Pose& is = side == 0 ? bs : cs;
+        const V3 rel = sub(is.x, rs.x);
+        for (uint32_t f = g.gl; f < rm.nt; f += kClipLanes) {
+            const float4 pl = rm.planes[f];
+            const V3 n = rotate(rs.q, v3(pl));
+            const V3 in = inv_rotate(is.q, n);
+            float support = kFltMax;
+            for (uint32_t k = 0; k < im.nv; ++k) support = fminf(support, dot(in, pv(im, k)));
+            const float sep = support + dot(n, rel) - pl.w;
+            if (sep > best) {
+                best = sep;
+                order = (side << 31) | f;
+            }
+        }
+    }
+    for (int o = kClipLanes / 2; o > 0; o >>= 1) {
+        const float v = __shfl_xor_sync(g.mask, best, o);
+        const uint32_t w = __shfl_xor_sync(g.mask, order, o);
+        if (v > best || (v == best && w < order)) {
+            best = v;
+            order = w;
+        }
+    }
+    if (order == 0xffffffffu) return {-kFltMax, 0u, false};  // no face separates (NaN): the serial start
+    return {best, order & 0x7fffffffu, (order >> 31) != 0};
+}
+
+// A manifold over the group: lane i < count holds contact i.
+struct LaneMan {
+    V3 normal, p;
+    float pen;
+    uint32_t count;
+};
+
+// add_contact (the contact is the same in every lane).
+__device__ __forceinline__ void add_contact_lanes(const LaneGroup& g, LaneMan& m, V3 p, float pen, float spacing) {
+    const float s2 = spacing * spacing;
+    const uint32_t near = g.ballot(g.gl < int(m.count) && len2(sub(m.p, p)) < s2);
+    int at = -1;
+    if (near) {
+        at = __ffs(near) - 1;
+        if (!(pen - g.from(m.pen, at) > 0.0f)) at = -1;
+    } else if (m.count < 8) {
+        at = int(m.count++);
+    } else {
+        float low = m.pen;  // the first of the shallowest
+        uint32_t who = uint32_t(g.gl);
+        for (int o = 4; o > 0; o >>= 1) {
+            const float v = __shfl_xor_sync(g.mask, low, o);
+            const uint32_t w = __shfl_xor_sync(g.mask, who, o);
+            if (v < low || (v == low && w < who)) {
+                low = v;
+                who = w;
+            }
+        }
+        who = g.from(who, 0);
+        if (pen > g.from(m.pen, int(who))) at = int(who);
+    }
+    if (g.gl == at) {
+        m.p = p;
+        m.pen = pen;
+    }
+}
+
+// reduce_face_patch: for each contact in turn, the 28 pairs of others in the
+// serial order, two rounds of 16.
+__device__ __forceinline__ void reduce_patch_lanes(const LaneGroup& g, LaneMan& m, float tol, ClipShared& sm) {
+    const float t2 = tol * tol;
+    for (uint32_t cand = 0; cand < m.count && m.count > 2;) {
+        __syncwarp(g.mask);
+        if (g.gl < int(m.count)) sm.man[g.gl] = f4(m.p, m.pen);
+        __syncwarp(g.mask);
+        const V3 p = v3(sm.man[cand]);
+        bool removed = false;
+        for (uint32_t r = 0; r < 2; ++r) {
+            uint32_t pair = uint32_t(g.gl) + 16u * r, f = 0;  // pairs f < s of 8, f-major
+            while (f < 7 && pair >= 7u - f) {
+                pair -= 7u - f;
+                ++f;
+            }
+            const uint32_t s = f + 1 + pair;
+            bool hit = f < 7 && s < m.count && f != cand && s != cand;
+            if (hit) {
+                const V3 pf = v3(sm.man[f]), e = sub(v3(sm.man[s]), pf);
+                const float e2 = len2(e);
+                hit = !(e2 <= t2);
+                if (hit) {
+                    const float par = dot(sub(p, pf), e) / e2;
+                    hit = !(par <= 1.0e-4f || par >= 0.9999f);
+                    if (hit) hit = !(len2(sub(p, add(pf, mul(e, par)))) > t2);
+                }
+            }
+            if (g.ballot(hit)) {
+                removed = true;
+                break;
+            }
+        }
+        if (!removed) {
+            ++cand;
+            continue;
+        }
+        // Contacts past it move down one; the search starts anew.
+        if (g.gl >= int(cand) && g.gl + 1 < int(m.count)) {
+            m.p = v3(sm.man[g.gl + 1]);
+            m.pen = sm.man[g.gl + 1].w;
+        }
+        --m.count;
+        cand = 0;
+    }
+}
+
+// face_manifold over the group; `outgrown`: a polygon needs more lanes.
+__device__ __forceinline__ bool face_manifold_lanes(const LaneGroup& g, const Pose& bs, const MeshRef& bm,
+                                                    const Pose& cs, const MeshRef& cm, float margin, float correction,
+                                                    LaneMan& out, const FaceSat& fs, ClipShared& sm, bool& outgrown) {
+    out.count = 0;
+    out.normal = out.p = {0, 0, 0};
+    out.pen = 0.0f;
+    const float rest = fmn(margin, 1.0e-3f);
+    const float reach = margin + correction;
+    if (fs.best > reach) return true;
+    const MeshRef& rm = fs.ref_body ? bm : cm;
+    const Pose& rs = fs.ref_body ? bs : cs;
+    const MeshRef& im = fs.ref_body ? cm : bm;
+    const Pose& is = fs.ref_body ? cs : bs;
+    const float4 ref = rm.planes[fs.ref_face];
+    const V3 refn = v3(ref);
+    const V3 outward = rotate(rs.q, refn);
+    const V3 inc_axis = inv_rotate(is.q, outward);
+    float align = 1.0f;
+    uint32_t inc_face = 0xffffffffu;
+    for (uint32_t f = g.gl; f < im.nt; f += kClipLanes) {
+        const float v = dot(inc_axis, v3(im.planes[f]));
+        if (v < align) {
+            align = v;
+            inc_face = f;
+        }
+    }
+    for (int o = kClipLanes / 2; o > 0; o >>= 1) {
+        const float v = __shfl_xor_sync(g.mask, align, o);
+        const uint32_t w = __shfl_xor_sync(g.mask, inc_face, o);
+        if (v < align || (v == align && w < inc_face)) {
+            align = v;
+            inc_face = w;
+        }
+    }
+    if (inc_face == 0xffffffffu) inc_face = 0;
+    out.normal = mul(outward, fs.ref_body ? -1.0f : 1.0f);
+    const float4 inc = im.planes[inc_face];
+    const float spacing = fmx(margin * 2.0f, 1.0e-4f);
+    int buf = 0;
+    for (uint32_t t0 = 0; t0 < im.nt; t0 += kClipLanes) {
+        bool facing = false;
+        if (t0 + g.gl < im.nt) {
+            const float4 face = im.planes[t0 + g.gl];
+            facing = !(dot(v3(face), v3(inc)) < 0.99999f || fab(face.w - inc.w) > 1.0e-5f);
+        }
+        for (uint32_t todo = g.ballot(facing); todo; todo &= todo - 1u) {
+            const uint32_t t = t0 + uint32_t(__ffs(todo) - 1);
+            // The incident triangle's corners in the reference body's frame.
+            int count = 3;
+            V3 cur{0, 0, 0};
+            if (g.gl < 3) {
+                const float4 packed = im.planes[im.nt + t];
+                const uint32_t idx = __float_as_uint(g.gl == 0 ? packed.x : g.gl == 1 ? packed.y : packed.z);
+                cur = inv_rotate(rs.q, sub(add(is.x, rotate(is.q, pv(im, idx))), rs.x));
+            }
+            for (uint32_t pi = 0; pi < rm.nt && count != 0; ++pi) {
+                const float4 pl = rm.planes[pi];
+                const V3 pn = v3(pl);
+                const float off = pl.w + (dot(pn, refn) > 0.99999f ? reach : 0.0f);
+                const float dd = dot(pn, cur) - off;
+                const int before = g.gl == 0 ? count - 1 : g.gl - 1;
+                const V3 prev{g.from(cur.x, before), g.from(cur.y, before), g.from(cur.z, before)};
+                const float pd = g.from(dd, before);
+                const bool live = g.gl < count;
+                const bool in = live && dd <= 0.0f, cross = live && (dd <= 0.0f) != (pd <= 0.0f);
+                const uint32_t ins = g.ballot(in), crosses = g.ballot(cross);
+                if (crosses == 0 && ins == (1u << count) - 1u) continue;  // nothing clipped
+                const int total = __popc(ins) + __popc(crosses);
+                if (total > kClipLanes) {
+                    outgrown = true;
+                    return false;
+                }
+                const uint32_t lower = (1u << g.gl) - 1u;
+                int at = __popc(ins & lower) + __popc(crosses & lower);
+                float4* dst = sm.poly[buf];
+                if (cross) dst[at++] = f4(add(prev, mul(sub(cur, prev), pd / (pd - dd))));
+                if (in) dst[at] = f4(cur);
+                __syncwarp(g.mask);
+                count = total;
+                if (g.gl < count) cur = v3(dst[g.gl]);
+                buf ^= 1;
+            }
+            const float dist = dot(refn, cur) - ref.w;
+            const V3 p = add(rs.x, rotate(rs.q, sub(cur, mul(refn, dist * 0.5f))));
+            const float pen = rest - dist + 1.0e-5f;
+            for (uint32_t k = g.ballot(g.gl < count && !(dist > reach)); k; k &= k - 1u) {
+                const int l = __ffs(k) - 1;
+                add_contact_lanes(g, out, V3{g.from(p.x, l), g.from(p.y, l), g.from(p.z, l)}, g.from(pen, l), spacing);
+            }
+        }
+    }
+    if (out.count == 0) return false;
+    reduce_patch_lanes(g, out, fmx(1.0e-6f, margin * 1.0e-3f), sm);
+    return true;
+}
+
+// The first part of swept_face_manifold: when the translating pair's faces
+// touch. kind 0: not a translation; 1: never (an empty manifold); 2: they
+// touch at the start; 3: at `entry`, along entry_n.
+struct SweptEntry {
+    int kind;
+    float entry;
+    V3 entry_n;
+};
+__device__ __forceinline__ SweptEntry swept_entry_lanes(const LaneGroup& g, const Pose& pb, const Pose& b,
+                                                        const MeshRef& bm, const Pose& pc, const Pose& c,
+                                                        const MeshRef& cm, float margin) {
+    const Q4 bd = qrelative(pb.q, b.q, false), cd = qrelative(pc.q, c.q, false);
+    if (bd.x != 0.0f || bd.y != 0.0f || bd.z != 0.0f || cd.x != 0.0f || cd.y != 0.0f || cd.z != 0.0f)
+        return {0, 0.0f, {0, 0, 0}};
+    const V3 bmo = sub(b.x, pb.x), cmo = sub(c.x, pc.x);
+    const float rest = fmn(margin, 1.0e-3f);
+    float entry = 0.0f, exit_t = 1.0f;
+    uint32_t order = 0xffffffffu;
+    V3 entry_n{0, 0, 0};
+    bool apart = false;
+    for (uint32_t side = 0; side < 2; ++side) {
+        const MeshRef& rm = side == 0 ? cm : bm;
+        const MeshRef& im = side == 0 ? bm : cm;
+        const Pose& rs = side == 0 ? pc : pb;
+        const Pose& is = side == 0 ? pb : pc;
+        const V3 rel = side == 0 ? sub(bmo, cmo) : sub(cmo, bmo);
+        for (uint32_t f = g.gl; f < rm.nt; f += kClipLanes) {
+            const float4 pl = rm.planes[f];
+            const V3 n = rotate(rs.q, v3(pl));
+            const V3 in = inv_rotate(is.q, n);
+            float support = kFltMax;
+            for (uint32_t k = 0; k < im.nv; ++k) support = fminf(support, dot(in, pv(im, k)));
+            const float gap = support + dot(n, sub(is.x, rs.x)) - pl.w;
+            const float speed = dot(n, rel);
+            if (speed == 0.0f) {
+                if (gap > rest) apart = true;
+            } else {
+                const float crossing = (rest - gap) / speed;
+                if (speed < 0.0f && crossing > entry) {
+                    entry = crossing;
+                    entry_n = mul(n, side == 0 ? 1.0f : -1.0f);
+                    order = (side << 31) | f;
+                }
+                if (speed > 0.0f) exit_t = fmn(exit_t, crossing);
+            }
+        }
+    }
+    if (g.ballot(apart)) return {1, 0.0f, {0, 0, 0}};
+    uint32_t who = uint32_t(g.gl);
+    for (int o = kClipLanes / 2; o > 0; o >>= 1) {
+        const float v = __shfl_xor_sync(g.mask, entry, o);
+        const uint32_t w = __shfl_xor_sync(g.mask, order, o), l = __shfl_xor_sync(g.mask, who, o);
+        if (v > entry || (v == entry && w < order)) {
+            entry = v;
+            order = w;
+            who = l;
+        }
+        exit_t = fmn(exit_t, __shfl_xor_sync(g.mask, exit_t, o));
+    }
+    who = g.from(who, 0);
+    entry_n = {g.from(entry_n.x, int(who)), g.from(entry_n.y, int(who)), g.from(entry_n.z, int(who))};
+    if (entry > exit_t || entry > 1.0f || exit_t < 0.0f) return {1, 0.0f, {0, 0, 0}};
+    return {entry == 0.0f ? 2 : 3, entry, entry_n};
+}
+
+// Where a candidate's pass 2 ends: its staged contacts, an empty manifold, or
+// the triangle-mesh path.
+__device__ __forceinline__ bool reserve_stage(const Dev& d, uint32_t k, uint32_t count, uint32_t& slot) {
+    slot = atomicAdd(&d.ctr->n_stage, count);
+    const bool fits = slot + count <= d.cap_stage;
+    if (!fits) atomicOr(&d.ctr->status, kStContactOverflow);
+    d.np_count[k] = fits ? count : 0u;
+    d.np_scan[k] = fits ? ((uint64_t(1) << 32) | count) : 0ull;
+    if (fits) d.np_stage[k] = slot;
+    return fits;
+}
+// One thread's face manifold of a candidate (swept variant first when the
+// pair moved more than its margin).
+__device__ __forceinline__ void narrow_serial(const Dev& d, uint32_t k, uint2 sat) {
+    const uint32_t a = d.cand_a[k], b = d.cand_b[k];
+    Man m;
+    m.count = 0;
+    const MeshRef bm = mesh_ref(d, d.mesh[a]), cm = mesh_ref(d, d.mesh[b]);
+    const CandidateMotion c = candidate_motion(d, a, b);
+    bool ok = false;
+    if (c.swept) ok = swept_face_manifold(c.prev_a, c.pred_a, bm, c.prev_b, c.pred_b, cm, c.margin, m);
+    if (!ok) {
+        // An unswept pair's separating-axis result comes from pass 1.
+        const FaceSat fs{__uint_as_float(sat.x), sat.y & 0x7fffffffu, (sat.y >> 31) != 0};
+        ok = face_manifold(c.pred_a, bm, c.pred_b, cm, c.margin, c.corr, m, c.swept ? nullptr : &fs);
+        if (c.swept && m.count == 0) ok = false;
+    }
+    if (!ok) {
+        declined(d, k, a, b);
+        return;
+    }
+    if (!m.count) {
+        d.np_count[k] = 0;
+        d.np_scan[k] = 0ull;
+        return;
+    }
+    uint32_t slot;
+    if (!reserve_stage(d, k, m.count, slot)) return;
+    for (uint32_t p = 0; p < m.count; ++p) {
+        d.st_n[slot + p] = f4(m.normal, m.pen[p]);
+        d.st_p[slot + p] = f4(m.p[p], m.impact);
+    }
+}
+
+// (Not inlined into the lanes' kernel, where it is rare.)
+__device__ __noinline__ void narrow_outgrown(const Dev& d, uint32_t k, uint2 sat) { narrow_serial(d, k, sat); }
+
+// Pass 2, a thread or 16 lanes per surviving candidate. With few survivors
+// the serial chain is what counts (217: 43 us with lanes, 124 with threads);
+// with many, the lanes' extra work (25,000: 176 and 190 us; 412,000: 2.36 and
+// 0.97 ms). The survivors' number is not known at the launch; piles have
+// about six a body, so worlds of up to kLaneBodies bodies take the lanes.
+constexpr uint32_t kLaneBodies = 3072;
 __global__ void __launch_bounds__(128, 6) k_narrow(Dev d) {
+    tick_begin();
     const uint32_t total = d.ctr->n_surv;
-    for (uint32_t s = grid_stride_begin(); s < total; s += grid_stride()) {
+    for (uint32_t s = grid_stride_begin(); s < total; s += grid_stride()) narrow_serial(d, d.np_list[s], d.np_sat[s]);
+}
+__global__ void __launch_bounds__(kNarrowThreads) k_narrow_lanes(const __grid_constant__ Dev d) {
+    tick_begin();
+    __shared__ ClipShared shared[kNarrowThreads / kClipLanes];
+    const uint32_t total = d.ctr->n_surv;
+    const int lane = threadIdx.x & 31, gl = lane % kClipLanes;
+    const LaneGroup g{0xffffu << (lane - gl), gl, lane - gl};
+    ClipShared& sm = shared[threadIdx.x / kClipLanes];
+    for (uint32_t s = grid_stride_begin() / kClipLanes; s < total; s += grid_stride() / kClipLanes) {
         const uint32_t k = d.np_list[s];
         const uint2 sat = d.np_sat[s];
         const uint32_t a = d.cand_a[k], b = d.cand_b[k];
-        const uint32_t ma = d.mesh[a], mb = d.mesh[b];
-        Man m;
-        m.count = 0;
-        const MeshRef bm = mesh_ref(d, ma), cm = mesh_ref(d, mb);
+        const MeshRef bm = mesh_ref(d, d.mesh[a]), cm = mesh_ref(d, d.mesh[b]);
         const CandidateMotion c = candidate_motion(d, a, b);
-        bool ok = false;
-        if (c.swept) ok = swept_face_manifold(c.prev_a, c.pred_a, bm, c.prev_b, c.pred_b, cm, c.margin, m);
-        if (!ok) {
-            // An unswept pair's separating-axis result comes from pass 1.
-            const FaceSat fs{__uint_as_float(sat.x), sat.y & 0x7fffffffu, (sat.y >> 31) != 0};
-            ok = face_manifold(c.pred_a, bm, c.pred_b, cm, c.margin, c.corr, m, c.swept ? nullptr : &fs);
-            if (c.swept && m.count == 0) ok = false;
-        }
-        if (!ok) {
-            // Most declined pairs lie beyond the pair margin: their root
-            // bounds (the mesh path's first test) settle them here.
-            if (mesh_pair_bounds_overlap(d, a, b, false)) {
-                to_mesh_path(d, k);
+        // The manifolds to try, in order. A translating pair that moved more
+        // than its margin: where it touches at the start, the predicted poses
+        // and then the previous ones; where it touches on the way, the poses
+        // then; failing those (and any other pair), the predicted poses with
+        // the correction.
+        enum { kNow, kStart, kEntry, kPlain };
+        SweptEntry se{0, 0.0f, {0, 0, 0}};
+        if (c.swept) se = swept_entry_lanes(g, c.prev_a, c.pred_a, bm, c.prev_b, c.pred_b, cm, c.margin);
+        int mode = se.kind == 2 ? kNow : se.kind == 3 ? kEntry : kPlain;
+        LaneMan m{{0, 0, 0}, {0, 0, 0}, 0.0f, 0u};
+        float impact = 1.0f;
+        bool ok = se.kind == 1, outgrown = false;
+        const V3 bmo = sub(c.pred_a.x, c.prev_a.x), cmo = sub(c.pred_b.x, c.prev_b.x);
+        const float rest = fmn(c.margin, 1.0e-3f);
+        while (!ok) {
+            Pose pa = c.pred_a, pb = c.pred_b;
+            if (mode == kStart) {
+                pa = c.prev_a;
+                pb = c.prev_b;
+            } else if (mode == kEntry) {
+                pa = {add(c.prev_a.x, mul(bmo, se.entry)), c.prev_a.q};
+                pb = {add(c.prev_b.x, mul(cmo, se.entry)), c.prev_b.q};
+            }
+            const FaceSat fs = !c.swept ? FaceSat{__uint_as_float(sat.x), sat.y & 0x7fffffffu, (sat.y >> 31) != 0}
+                                        : face_sat_lanes(g, pa, bm, pb, cm);
+            const bool clipped =
+                face_manifold_lanes(g, pa, bm, pb, cm, mode == kEntry ? rest + 1.0e-5f : c.margin,
+                                    mode == kPlain ? c.corr : 0.0f, m, fs, sm, outgrown);
+            if (outgrown) break;
+            impact = 1.0f;
+            if (mode == kPlain) {
+                ok = clipped && !(c.swept && m.count == 0);
+                break;
+            }
+            const bool some = clipped && m.count != 0;
+            if (mode == kNow) {
+                ok = some;
+                mode = kStart;
+            } else if (mode == kStart) {
+                const float closing = -dot(sub(bmo, cmo), m.normal);
+                if (some && !(closing <= 0.0f)) {
+                    m.pen += closing;
+                    impact = 0.0f;
+                    ok = true;
+                }
+                mode = kPlain;
             } else {
+                if (some && !(dot(m.normal, se.entry_n) < 0.99999f)) {
+                    const float remaining = -dot(sub(bmo, cmo), m.normal) * (1.0f - se.entry);
+                    m.pen = fmx(0.0f, remaining + m.pen) + rest + 1.0e-5f;
+                    impact = se.entry;
+                    ok = true;
+                }
+                mode = kPlain;
+            }
+        }
+        if (outgrown) {
+            if (gl == 0) narrow_outgrown(d, k, sat);
+        } else if (!ok) {
+            if (gl == 0) declined(d, k, a, b);
+        } else if (m.count == 0) {
+            if (gl == 0) {
                 d.np_count[k] = 0;
                 d.np_scan[k] = 0ull;
             }
-            continue;
-        }
-        const uint32_t count = m.count;
-        d.np_count[k] = count;
-        d.np_scan[k] = count ? ((uint64_t(1) << 32) | count) : 0ull;
-        if (count) {
-            uint32_t slot = atomicAdd(&d.ctr->n_stage, count);
-            if (slot + count > d.cap_stage) {
-                atomicOr(&d.ctr->status, kStContactOverflow);
-                d.np_scan[k] = 0ull;
-                d.np_count[k] = 0;
-                continue;
-            }
-            d.np_stage[k] = slot;
-            for (uint32_t p = 0; p < count; ++p) {
-                d.st_n[slot + p] = f4(m.normal, m.pen[p]);
-                d.st_p[slot + p] = f4(m.p[p], m.impact);
+        } else {
+            uint32_t slot = 0, fits = 0;
+            if (gl == 0) fits = reserve_stage(d, k, m.count, slot) ? 1u : 0u;
+            slot = g.from(slot, 0);
+            if (g.from(fits, 0) && gl < int(m.count)) {
+                d.st_n[slot + gl] = f4(m.normal, m.pen);
+                d.st_p[slot + gl] = f4(m.p, impact);
             }
         }
+        __syncwarp(g.mask);
     }
 }
 
 // Scatter non-empty manifolds to their pair-ordered place and finalize them
 // (geometry.slang:2852-2872: initial normal speed from predicted velocities).
 __global__ void k_compact(Dev d) {
+    tick_begin();
     const uint32_t total = d.ctr->n_cand;
     const uint64_t grand = d.np_scan[total];
     const uint32_t n_act = uint32_t(grand >> 32), n_con = uint32_t(grand & 0xffffffffu);
@@ -457,6 +879,7 @@ __global__ void k_compact(Dev d) {
 // geometry.slang:2941-3009, keyed by pair code against the previous tick's
 // sorted saved pairs.
 __global__ void k_cache_load(Dev d, StepParams sp) {
+    tick_begin();
     const uint32_t n_act = d.ctr->n_act;
     const uint32_t n_saved = *d.sv_n_pairs;
     const float dt = sp.dt;
@@ -511,20 +934,21 @@ __global__ void k_cache_load(Dev d, StepParams sp) {
 }
 
 void launch_narrowphase(const Dev& d, const StepParams& sp, cudaStream_t s) {
-    k_narrow_sat<<<cap_blocks(d.cap_cand, 256), 256, 0, s>>>(d);
-    note_launch(cap_blocks(d.cap_cand, 256));
+    launch(k_narrow_sat, cap_blocks(d.cap_cand, 256), 256, s, d);
     prof_mark(s, "narrowphase SAT");
-    k_narrow<<<cap_blocks(d.cap_cand, 128), 128, 0, s>>>(d);
-    note_launch(cap_blocks(d.cap_cand, 128));
+    if (d.n <= kLaneBodies) {
+        const uint32_t grid = cap_blocks(size_t(kClipLanes) * d.cap_cand, kNarrowThreads);
+        launch(k_narrow_lanes, grid, kNarrowThreads, s, d);
+    } else {
+        launch(k_narrow, cap_blocks(d.cap_cand, 128), 128, s, d);
+    }
     prof_mark(s, "narrowphase manifolds");
     launch_mesh_narrowphase(d, sp, s);
     prof_mark(s, "narrowphase meshes");
     scan_u64(d.np_scan, d.np_scan, &d.ctr->n_cand, d.cap_cand, d.scan_tmp, s);
-    k_compact<<<cap_blocks(d.cap_cand), kBlock, 0, s>>>(d);
-    note_launch(cap_blocks(d.cap_cand));
+    launch(k_compact, cap_blocks(d.cap_cand), kBlock, s, d);
     prof_mark(s, "compact");
-    k_cache_load<<<cap_blocks(d.cap_pair, 128), 128, 0, s>>>(d, sp);
-    note_launch(cap_blocks(d.cap_pair, 128));
+    launch(k_cache_load, cap_blocks(d.cap_pair, 128), 128, s, d, sp);
     prof_mark(s, "cache load");
 }
 

@@ -174,11 +174,13 @@ __device__ __forceinline__ void prepare_pairs(const Dev& d, const StepParams& sp
 
 // (Pairs read nothing that the bodies' part writes.)
 __global__ void __launch_bounds__(128) k_prepare(Dev d, StepParams sp) {
+    tick_begin();
     prepare_bodies(d, sp);
     prepare_pairs(d, sp);
 }
 
 __global__ void k_prepare_joints(Dev d, StepParams sp) {
+    tick_begin();
     const float dt = sp.dt;
     for (uint32_t j = grid_stride_begin(); j < d.nj; j += grid_stride()) {
         JointState st = d.jstate[j];
@@ -239,6 +241,7 @@ __device__ void uf_unite(uint32_t* parent, uint32_t a, uint32_t b) {
 // The incidence counts and unions, and each contact's record of the position
 // phase (which only the sweeps read).
 __global__ void k_graph_degrees(Dev d, StepParams sp) {
+    tick_begin();
     const uint32_t n_con = d.ctr->n_contacts;
     for (uint32_t c = grid_stride_begin(); c < n_con; c += grid_stride()) {
         const uint2 ab = d.c_bodies[c];
@@ -275,6 +278,7 @@ __global__ void k_graph_degrees(Dev d, StepParams sp) {
 // budget raised by the scene's largest joint iteration hint. Also clears the
 // scene's residual accumulators and joint hints for the next tick.
 __global__ void k_scene_budgets(Dev d, StepParams sp) {
+    tick_begin();
     for (uint32_t s = grid_stride_begin(); s < d.n_scenes; s += grid_stride()) {
         const uint32_t req = d.scene_iters[s] ? d.scene_iters[s] : sp.requested;
         uint32_t budget = sp.realtime ? 8u : (req ? req : sp.budget_request);
@@ -290,11 +294,11 @@ __global__ void k_scene_budgets(Dev d, StepParams sp) {
 }
 void launch_scene_budgets(const Dev& d, const StepParams& sp, cudaStream_t s) {
     if (d.n_scenes <= 1) return;
-    k_scene_budgets<<<blocks_for(d.n_scenes), kBlock, 0, s>>>(d, sp);
-    note_launch(blocks_for(d.n_scenes));
+    launch(k_scene_budgets, blocks_for(d.n_scenes), kBlock, s, d, sp);
 }
 
 __global__ void k_graph_fill(Dev d) {
+    tick_begin();
     const uint32_t n_act = d.ctr->n_act;
     for (uint32_t i = grid_stride_begin(); i < n_act; i += grid_stride()) {
         const uint32_t a = d.act_a[i], b = d.act_b[i];
@@ -325,6 +329,7 @@ __device__ __forceinline__ void sort_desc(uint32_t* seg, uint32_t n) {
 // (writing ancestors), so roots go to a scratch array (corder, refilled by the
 // colour pass later) and are published by a second kernel.
 __global__ void k_graph_lists(Dev d) {
+    tick_begin();
     for (uint32_t i = grid_stride_begin(); i < d.n; i += grid_stride()) {
         sort_desc(d.inc_list + d.inc_off[i], d.deg[i]);
         sort_desc(d.jinc_list + d.jinc_off[i], d.jdeg[i]);
@@ -332,6 +337,7 @@ __global__ void k_graph_lists(Dev d) {
     }
 }
 __global__ void k_graph_roots(Dev d) {
+    tick_begin();
     for (uint32_t i = grid_stride_begin(); i < d.n; i += grid_stride()) {
         d.parent[i] = d.corder[i];
         uint32_t rc = 0;
@@ -428,6 +434,7 @@ __device__ __forceinline__ void neighbour_lists(const Dev& d) {
 // What the sorted lists and the roots give: contact rows, neighbours, impact
 // marks at the islands' roots.
 __global__ void k_graph_rows(Dev d) {
+    tick_begin();
     row_lists(d);
     neighbour_lists(d);
     graph_impact(d);
@@ -553,6 +560,7 @@ __device__ __forceinline__ void color_offsets(const Dev& d, uint32_t* count) {
 // bodies, where the launches cost more than the block's few rounds.
 constexpr uint32_t kOneBlockOrder = 8192;
 __global__ void k_color_count(Dev d) {
+    tick_begin();
     graph_islands(d);
     for (uint32_t i = grid_stride_begin(); i < d.n; i += grid_stride()) {
         if (d.motion[i] != kDynamic) continue;
@@ -560,8 +568,10 @@ __global__ void k_color_count(Dev d) {
         atomicMax(&d.ctr->colors, d.color[i] + 1);
     }
 }
-__global__ void __launch_bounds__(1024) k_color_offsets(Dev d) { color_offsets(d, d.ctr->color_count); }
+__global__ void __launch_bounds__(1024) k_color_offsets(Dev d) {
+    tick_begin(); color_offsets(d, d.ctr->color_count); }
 __global__ void k_color_scatter(Dev d) {
+    tick_begin();
     for (uint32_t i = grid_stride_begin(); i < d.n; i += grid_stride()) {
         if (d.motion[i] != kDynamic) continue;
         const uint32_t b = color_bucket(d, i);
@@ -569,6 +579,7 @@ __global__ void k_color_scatter(Dev d) {
     }
 }
 __global__ void __launch_bounds__(1024) k_color_order(Dev d) {
+    tick_begin();
     __shared__ uint32_t count[kBuckets];
     __shared__ uint32_t colors;
     for (uint32_t b = threadIdx.x; b < kBuckets; b += blockDim.x) count[b] = 0;
@@ -593,11 +604,9 @@ __global__ void __launch_bounds__(1024) k_color_order(Dev d) {
 
 void launch_prepare(const Dev& d, const StepParams& sp, cudaStream_t s) {
     const uint32_t grid = cap_blocks(std::max(d.cap_pair, d.n), 128);
-    k_prepare<<<grid, 128, 0, s>>>(d, sp);
-    note_launch(grid);
+    launch(k_prepare, grid, 128, s, d, sp);
     if (d.nj) {
-        k_prepare_joints<<<blocks_for(d.nj, 64), 64, 0, s>>>(d, sp);
-        note_launch(blocks_for(d.nj, 64));
+        launch(k_prepare_joints, blocks_for(d.nj, 64), 64, s, d, sp);
     }
     prof_mark(s, "prepare");
 }
@@ -607,39 +616,30 @@ const void* color_kernel_ptr = reinterpret_cast<const void*>(&k_color);
 void launch_graph(const Dev& d, const StepParams& sp, cudaStream_t s, int coop_blocks) {
     uint32_t gb = cap_blocks(d.cap_pair > d.nj ? d.cap_pair : d.nj);
     const uint32_t db = cap_blocks(std::max({d.cap_pair, d.nj, d.cap_contact}));
-    k_graph_degrees<<<db, kBlock, 0, s>>>(d, sp);
-    note_launch(db);
+    launch(k_graph_degrees, db, kBlock, s, d, sp);
     // (Without joints the joint lists' offsets stay the zeros of the world's
     // creation.)
     if (d.nj)
         scan_u32_pair(d.deg, d.inc_off, nullptr, d.jdeg, d.jinc_off, nullptr, nullptr, d.n, d.scan_tmp32, s);
     else
         scan_u32(d.deg, d.inc_off, nullptr, d.n, nullptr, 0u, d.scan_tmp32, s);
-    k_graph_fill<<<gb, kBlock, 0, s>>>(d);
-    note_launch(gb);
-    k_graph_lists<<<blocks_for(d.n), kBlock, 0, s>>>(d);
-    note_launch(blocks_for(d.n));
-    k_graph_roots<<<blocks_for(d.n), kBlock, 0, s>>>(d);
-    note_launch(blocks_for(d.n));
+    launch(k_graph_fill, gb, kBlock, s, d);
+    launch(k_graph_lists, blocks_for(d.n), kBlock, s, d);
+    launch(k_graph_roots, blocks_for(d.n), kBlock, s, d);
     scan_u32(d.rcount, d.roff, nullptr, d.n, nullptr, 0u, d.scan_tmp32, s);
     const uint32_t rb = cap_blocks(std::max(d.cap_pair, d.n));
-    k_graph_rows<<<rb, kBlock, 0, s>>>(d);
-    note_launch(rb);
+    launch(k_graph_rows, rb, kBlock, s, d);
     prof_mark(s, "graph lists");
     void* args[] = {const_cast<Dev*>(&d)};
     cudaLaunchCooperativeKernel(color_kernel_ptr, dim3(coop_blocks), dim3(kColorThreads), args, 0, s);
     note_launch(coop_blocks);
     prof_mark(s, "colour fixpoint");
     if (d.n <= kOneBlockOrder) {
-        k_color_order<<<1, 1024, 0, s>>>(d);
-        note_launch(1);
+        launch(k_color_order, 1, 1024, s, d);
     } else {
-        k_color_count<<<blocks_for(d.n), kBlock, 0, s>>>(d);
-        note_launch(blocks_for(d.n));
-        k_color_offsets<<<1, 1024, 0, s>>>(d);
-        note_launch(1);
-        k_color_scatter<<<blocks_for(d.n), kBlock, 0, s>>>(d);
-        note_launch(blocks_for(d.n));
+        launch(k_color_count, blocks_for(d.n), kBlock, s, d);
+        launch(k_color_offsets, 1, 1024, s, d);
+        launch(k_color_scatter, blocks_for(d.n), kBlock, s, d);
     }
     prof_mark(s, "islands+colour order");
 }

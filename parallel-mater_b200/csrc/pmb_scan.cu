@@ -81,6 +81,7 @@ template <class T> struct ScanJobs {
 template <class T>
 __global__ void __launch_bounds__(kScanBlockThreads)
     k_scan_block(ScanJobs<T> jobs, const uint32_t* count_ptr, uint32_t capacity, uint32_t total_cap) {
+    tick_begin();
     const T* in = jobs.job[blockIdx.y].in;
     T* out = jobs.job[blockIdx.y].out;
     T* total = jobs.job[blockIdx.y].total;
@@ -103,6 +104,7 @@ __global__ void __launch_bounds__(kScanBlockThreads)
 
 template <class T>
 __global__ void k_tile_sums(ScanJobs<T> jobs, const uint32_t* count_ptr, uint32_t capacity) {
+    tick_begin();
     const T* in = jobs.job[blockIdx.y].in;
     T* tile_sums = jobs.job[blockIdx.y].tiles;
     const uint32_t count = count_ptr ? min(*count_ptr, capacity) : capacity;
@@ -117,6 +119,7 @@ __global__ void k_tile_sums(ScanJobs<T> jobs, const uint32_t* count_ptr, uint32_
 
 template <class T>
 __global__ void k_scan_apply(ScanJobs<T> jobs, const uint32_t* count_ptr, uint32_t capacity, uint32_t total_cap) {
+    tick_begin();
     const T* in = jobs.job[blockIdx.y].in;
     T* out = jobs.job[blockIdx.y].out;
     T* total = jobs.job[blockIdx.y].total;
@@ -147,15 +150,12 @@ template <class T>
 static void scan_impl(const ScanJobs<T>& jobs, uint32_t njobs, const uint32_t* count_ptr, uint32_t capacity,
                       uint32_t total_cap, cudaStream_t s) {
     if (capacity <= kScanBlockMost) {
-        k_scan_block<T><<<dim3(1, njobs), kScanBlockThreads, 0, s>>>(jobs, count_ptr, capacity, total_cap);
-        note_launch(njobs);
+        launch(k_scan_block<T>, dim3(1, njobs), kScanBlockThreads, s, jobs, count_ptr, capacity, total_cap);
         return;
     }
     const uint32_t tiles = (capacity + kScanTile - 1) / kScanTile;
-    k_tile_sums<T><<<dim3(tiles, njobs), kScanThreads, 0, s>>>(jobs, count_ptr, capacity);
-    note_launch(tiles * njobs);
-    k_scan_apply<T><<<dim3(tiles, njobs), kScanThreads, 0, s>>>(jobs, count_ptr, capacity, total_cap);
-    note_launch(tiles * njobs);
+    launch(k_tile_sums<T>, dim3(tiles, njobs), kScanThreads, s, jobs, count_ptr, capacity);
+    launch(k_scan_apply<T>, dim3(tiles, njobs), kScanThreads, s, jobs, count_ptr, capacity, total_cap);
 }
 
 void scan_u32(const uint32_t* in, uint32_t* out, const uint32_t* count_ptr, uint32_t capacity, uint32_t* total,

@@ -22,6 +22,7 @@ namespace pmb {
 // forces less them) -- the normal impulse and the accumulated friction of the
 // position phase, both fixed by then, over dt -- and the joints' rows.
 __global__ void k_impact_rows(Dev d, float dt, const float4* ov, const float4* ow) {
+    tick_begin();
     if (d.ctr->impact == 0) return;
     for (uint32_t j = grid_stride_begin(); j < d.nj; j += grid_stride()) {
         const JointState st = d.jstate[j];
@@ -779,6 +780,7 @@ __device__ __forceinline__ void free_anchor(const Dev& d) {
 
 // Both need only the solved displacements.
 __global__ void k_finish_contacts(Dev d, StepParams sp, uint32_t phase) {
+    tick_begin();
     if (phase != 0 && d.ctr->impact == 0) return;
     contact_finalize(d, sp, phase);
     free_anchor(d);
@@ -790,6 +792,7 @@ __global__ void k_finish_contacts(Dev d, StepParams sp, uint32_t phase) {
 // root loop (geometry_constraints_solve.slang:617-698) without its scan over
 // all bodies.
 __global__ void k_free_mean(Dev d, uint32_t phase) {
+    tick_begin();
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, warps = (gridDim.x * blockDim.x) >> 5;
     for (uint32_t r = warp; r < d.n; r += warps) {
@@ -826,6 +829,7 @@ __global__ void k_free_mean(Dev d, uint32_t phase) {
 // The free islands' means taken off, then apply_states
 // (geometry_constraints_solve.slang:676-733) into the output state arrays (v: solved state; t: the AVBD target stays untouched).
 __global__ void k_apply(Dev d, StepParams sp, uint32_t phase, float4* ox, float4* oq, float4* ov, float4* ow) {
+    tick_begin();
     if (phase != 0 && d.ctr->impact == 0) return;
     const float dt = sp.dt;
     for (uint32_t i = grid_stride_begin(); i < d.n; i += grid_stride()) {
@@ -870,6 +874,7 @@ __global__ void k_apply(Dev d, StepParams sp, uint32_t phase, float4* ox, float4
 // serial over the hinge joints in index order, as in the reference. One
 // thread per scene segment (scenes of a batched world share no bodies).
 __global__ void k_project_hinges(Dev d, float4* ox, const float4* oq) {
+    tick_begin();
     const uint32_t seg = blockIdx.x * blockDim.x + threadIdx.x;
     if (seg >= d.n_hinge_segs) return;
     for (uint32_t h = d.hinge_seg[seg]; h < d.hinge_seg[seg + 1]; ++h) {
@@ -893,6 +898,7 @@ __global__ void k_project_hinges(Dev d, float4* ox, const float4* oq) {
 // Velocity-phase setup (geometry_constraints_solve.slang:238-330).
 __global__ void k_impact_setup(Dev d, StepParams sp, const float4* ox, const float4* oq, const float4* ov,
                                const float4* ow) {
+    tick_begin();
     if (d.ctr->impact == 0) return;
     const uint32_t n_act = d.ctr->n_act;
     // impact_gaps (uses the phase-0 displacements)
@@ -910,6 +916,7 @@ __global__ void k_impact_setup(Dev d, StepParams sp, const float4* ox, const flo
     }
 }
 __global__ void k_impact_bodies(Dev d, const float4* ox, const float4* oq, const float4* ov, const float4* ow) {
+    tick_begin();
     if (d.ctr->impact == 0) return;
     for (uint32_t i = grid_stride_begin(); i < d.n; i += grid_stride()) {
         if (d.impact[i] != 0 || d.motion[i] != kDynamic) {
@@ -929,6 +936,7 @@ __global__ void k_impact_bodies(Dev d, const float4* ox, const float4* oq, const
 // pair code (already sorted).
 __global__ void k_commit(Dev d, StepParams sp, const float4* ox, const float4* oq, const float4* ov,
                          const float4* ow) {
+    tick_begin();
     for (uint32_t i = grid_stride_begin(); i < d.n; i += grid_stride()) {
         V3 v = v3(ov[i]), w = v3(ow[i]);
         if (d.motion[i] == kDynamic) {
@@ -973,6 +981,7 @@ __global__ void k_commit(Dev d, StepParams sp, const float4* ox, const float4* o
 // normals and penetrations are the narrowphase's (unchanged since); the
 // impulses are those the cache save stores (convex pairs are persistent).
 __global__ void k_contact_events(Dev d) {
+    tick_begin();
     const uint32_t n = min(d.ctr->n_contacts, d.event_capacity);
     if (grid_stride_begin() == 0) d.ctr->n_events = n;
     for (uint32_t c = grid_stride_begin(); c < n; c += grid_stride()) {
@@ -1005,12 +1014,9 @@ void launch_solve_all(const Dev& d, const StepParams& sp, cudaStream_t s, int co
     const uint32_t fb = cap_blocks(std::max({d.cap_contact, d.cap_pair, d.n, d.nj}));
     for (uint32_t phase = 0; phase < (sp.realtime ? 1u : 2u); ++phase) {
         if (phase != 0) {
-            k_impact_setup<<<cap_blocks(d.cap_pair), kBlock, 0, s>>>(d, sp, o.ox, o.oq, o.ov, o.ow);
-            note_launch(cap_blocks(d.cap_pair));
-            k_impact_bodies<<<blocks_for(d.n), kBlock, 0, s>>>(d, o.ox, o.oq, o.ov, o.ow);
-            note_launch(blocks_for(d.n));
-            k_impact_rows<<<pb, kBlock, 0, s>>>(d, sp.dt, o.ov, o.ow);
-            note_launch(pb);
+            launch(k_impact_setup, cap_blocks(d.cap_pair), kBlock, s, d, sp, o.ox, o.oq, o.ov, o.ow);
+            launch(k_impact_bodies, blocks_for(d.n), kBlock, s, d, o.ox, o.oq, o.ov, o.ow);
+            launch(k_impact_rows, pb, kBlock, s, d, sp.dt, o.ov, o.ow);
             prof_mark(s, "impact setup");
         }
         Dev dd = d;
@@ -1025,24 +1031,18 @@ void launch_solve_all(const Dev& d, const StepParams& sp, cudaStream_t s, int co
         note_launch(coop);
         solve_timer_end(s);
         prof_mark(s, phase ? "solve phase 1" : "solve phase 0");
-        k_finish_contacts<<<fb, kBlock, 0, s>>>(d, sp, phase);
-        note_launch(fb);
-        k_free_mean<<<std::min<uint32_t>(blocks_for(32u * d.n, 256), 148u * 8u), 256, 0, s>>>(d, phase);
-        note_launch(std::min<uint32_t>(blocks_for(32u * d.n, 256), 148u * 8u));
-        k_apply<<<blocks_for(d.n), kBlock, 0, s>>>(d, sp, phase, o.ox, o.oq, o.ov, o.ow);
-        note_launch(blocks_for(d.n));
+        launch(k_finish_contacts, fb, kBlock, s, d, sp, phase);
+        launch(k_free_mean, std::min<uint32_t>(blocks_for(32u * d.n, 256), 148u * 8u), 256, s, d, phase);
+        launch(k_apply, blocks_for(d.n), kBlock, s, d, sp, phase, o.ox, o.oq, o.ov, o.ow);
         if (phase == 0 && d.n_hinge_segs) {
-            k_project_hinges<<<blocks_for(d.n_hinge_segs), kBlock, 0, s>>>(d, o.ox, o.oq);
-            note_launch(blocks_for(d.n_hinge_segs));
+            launch(k_project_hinges, blocks_for(d.n_hinge_segs), kBlock, s, d, o.ox, o.oq);
         }
         prof_mark(s, phase ? "finish phase 1" : "finish phase 0");
     }
     set_phase(kPhCommit);
-    k_commit<<<nb, kBlock, 0, s>>>(d, sp, o.ox, o.oq, o.ov, o.ow);
-    note_launch(nb);
+    launch(k_commit, nb, kBlock, s, d, sp, o.ox, o.oq, o.ov, o.ow);
     if (sp.collect_events && d.event_capacity) {
-        k_contact_events<<<cap_blocks(d.event_capacity), kBlock, 0, s>>>(d);
-        note_launch(cap_blocks(d.event_capacity));
+        launch(k_contact_events, cap_blocks(d.event_capacity), kBlock, s, d);
     }
     prof_mark(s, "commit+cache save");
 }

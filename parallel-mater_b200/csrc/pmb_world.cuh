@@ -14,6 +14,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include <utility>
+
 #include "pmb_math.cuh"
 
 namespace pmb {
@@ -444,6 +446,33 @@ void launch_mlp_apply(const Dev& d, const MlpMeta* meta, const float* out, uint3
                       cudaStream_t s);
 void launch_mlp_reduce_adam(const float* partial, uint32_t parts, float* grad, float* params, float* m, float* v,
                             float lr, float b1, float b2, float c1, float c2, float eps, float* gate, cudaStream_t s);
+
+// A tick is a chain of some 48 kernels, most of a few microseconds, and each
+// launch waited for the whole of the one before: about 1.5 us a step from one
+// kernel's end to the next one's first instruction. The kernels are launched
+// as programmatic dependents instead: a kernel lets the next one be set up
+// as soon as it runs itself, and every kernel waits at its top, in every
+// thread, for all memory of the kernels before it (tick_begin). So a kernel
+// that goes through launch() starts with tick_begin(); launched in any other
+// way, the call does nothing.
+__device__ __forceinline__ void tick_begin() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <class... P, class... A>
+inline void launch(void (*kernel)(P...), dim3 grid, uint32_t threads, cudaStream_t s, A&&... args) {
+    cudaLaunchConfig_t config{};
+    config.gridDim = grid;
+    config.blockDim = dim3(threads);
+    config.stream = s;
+    cudaLaunchAttribute attribute{};
+    attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attribute.val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = &attribute;
+    config.numAttrs = 1;
+    cudaLaunchKernelEx(&config, kernel, std::forward<A>(args)...);
+    note_launch(uint64_t(grid.x) * grid.y);
+}
 
 inline uint32_t blocks_for(uint32_t n, int threads = kBlock) {
     uint32_t b = (n + threads - 1) / threads;
