@@ -154,36 +154,66 @@ __device__ bool segment_hits_triangle(V3 p, V3 q, const Tri& t, V3& hit) {
            dot(cross(sub(t.v[0], t.v[2]), sub(hit, t.v[2])), n) >= tol;
 }
 
-// geometry.slang:1057-1105
-__device__ __noinline__ void closest_triangle_pair(const Tri& A, const Tri& B, V3& best_a, V3& best_b) {
+// geometry.slang:1057-1105. The triangles turn under the loops (v0, v1, v2 ->
+// v1, v2, v0) instead of being indexed by them: an index would put them in
+// local memory, and this is called up to 33 times for a triangle pair. By
+// value, and not inlined: inlining made the callers slower by their size.
+__device__ __forceinline__ void turn(Tri& t) {
+    const V3 v = t.v[0];
+    t.v[0] = t.v[1];
+    t.v[1] = t.v[2];
+    t.v[2] = v;
+}
+struct ClosestPair { V3 a, b; };
+__device__ __noinline__ ClosestPair closest_triangle_pair(Tri A, Tri B) {
+    ClosestPair r{{0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f}};
     V3 hit;
-    for (uint32_t e = 0; e < 3; ++e)
-        if (segment_hits_triangle(A.v[e], A.v[(e + 1) % 3], B, hit)) {
-            best_a = best_b = hit;
-            return;
+#pragma unroll 1
+    for (uint32_t side = 0; side < 2; ++side) {
+        // A's edges against B, then B's against A.
+#pragma unroll 1
+        for (uint32_t e = 0; e < 3; ++e) {
+            if (segment_hits_triangle(A.v[0], A.v[1], B, hit)) {
+                r.a = r.b = hit;
+                return r;
+            }
+            turn(A);
         }
-    for (uint32_t e = 0; e < 3; ++e)
-        if (segment_hits_triangle(B.v[e], B.v[(e + 1) % 3], A, hit)) {
-            best_a = best_b = hit;
-            return;
-        }
+        const Tri t = A;
+        A = B;
+        B = t;
+    }
     float best = 3.402823466e+38f;
     auto consider = [&](V3 p, V3 q) {
         const float s = len2(sub(p, q));
         if (s < best) {
             best = s;
-            best_a = p;
-            best_b = q;
+            r.a = p;
+            r.b = q;
         }
     };
-    for (uint32_t i = 0; i < 3; ++i) consider(A.v[i], closest_on_triangle(A.v[i], B.v[0], B.v[1], B.v[2]));
-    for (uint32_t i = 0; i < 3; ++i) consider(closest_on_triangle(B.v[i], A.v[0], A.v[1], A.v[2]), B.v[i]);
-    for (uint32_t i = 0; i < 3; ++i)
+#pragma unroll 1
+    for (uint32_t i = 0; i < 3; ++i) {
+        consider(A.v[0], closest_on_triangle(A.v[0], B.v[0], B.v[1], B.v[2]));
+        turn(A);
+    }
+#pragma unroll 1
+    for (uint32_t i = 0; i < 3; ++i) {
+        consider(closest_on_triangle(B.v[0], A.v[0], A.v[1], A.v[2]), B.v[0]);
+        turn(B);
+    }
+#pragma unroll 1
+    for (uint32_t i = 0; i < 3; ++i) {
+#pragma unroll 1
         for (uint32_t j = 0; j < 3; ++j) {
             V3 on_a, on_b;
-            closest_segments(A.v[i], A.v[(i + 1) % 3], B.v[j], B.v[(j + 1) % 3], on_a, on_b);
+            closest_segments(A.v[0], A.v[1], B.v[0], B.v[1], on_a, on_b);
             consider(on_a, on_b);
+            turn(B);
         }
+        turn(A);
+    }
+    return r;
 }
 
 // geometry.slang:1272-1290
@@ -244,39 +274,42 @@ __device__ bool point_inside_convex(const MeshView& m, const MeshPose& s, V3 p) 
 }
 
 // geometry.slang:1855-1908
-__device__ __noinline__ V3 triangle_feature_normal(const Tri& A, const Tri& B, V3 pa, V3 pb, V3 fallback) {
+__device__ __noinline__ V3 triangle_feature_normal(Tri A, Tri B, V3 pa, V3 pb, V3 fallback) {
     const V3 delta = sub(pa, pb);
     V3 n = normalized_or(delta, fallback);
-    const V3 faces[2] = {normalized_or(cross(sub(A.v[1], A.v[0]), sub(A.v[2], A.v[0])), n),
-                         normalized_or(cross(sub(B.v[1], B.v[0]), sub(B.v[2], B.v[0])), n)};
-    const Tri* tri[2] = {&A, &B};
-    const V3 pts[2] = {pa, pb};
+    const V3 face_a = normalized_or(cross(sub(A.v[1], A.v[0]), sub(A.v[2], A.v[0])), n);
+    const V3 face_b = normalized_or(cross(sub(B.v[1], B.v[0]), sub(B.v[2], B.v[0])), n);
     float align_best = -1.0f;
     V3 interior_n{0.0f, 0.0f, 0.0f};
+#pragma unroll
     for (uint32_t side = 0; side < 2; ++side) {
-        const Tri& t = *tri[side];
+        const Tri& t = side == 0 ? A : B;
+        const V3 pt = side == 0 ? pa : pb, face = side == 0 ? face_a : face_b;
         const V3 raw = cross(sub(t.v[1], t.v[0]), sub(t.v[2], t.v[0]));
         const float tol = 1.0e-5f * len2(raw);
         bool interior = tol > 0.0f;
+#pragma unroll
         for (uint32_t e = 0; e < 3; ++e)
-            interior = interior && dot(cross(sub(t.v[(e + 1) % 3], t.v[e]), sub(pts[side], t.v[e])), raw) > tol;
-        const float align = fab(dot(faces[side], n));
+            interior = interior && dot(cross(sub(t.v[(e + 1) % 3], t.v[e]), sub(pt, t.v[e])), raw) > tol;
+        const float align = fab(dot(face, n));
         if (interior && align > align_best) {
             align_best = align;
-            const float proj = dot(delta, faces[side]);
-            const float dir = fab(proj) > kEps ? proj : dot(fallback, faces[side]);
-            interior_n = dir >= 0.0f ? faces[side] : mul(faces[side], -1.0f);
+            const float proj = dot(delta, face);
+            const float dir = fab(proj) > kEps ? proj : dot(fallback, face);
+            interior_n = dir >= 0.0f ? face : mul(face, -1.0f);
         }
     }
     if (align_best >= 0.0f) return interior_n;
     float best_err = 4.0f * kEps * kEps;
     if (len2(delta) > kEps * kEps)
+#pragma unroll
         for (uint32_t side = 0; side < 2; ++side) {
-            const float proj = dot(delta, faces[side]);
-            const float err = len2(sub(delta, mul(faces[side], proj)));
+            const V3 face = side == 0 ? face_a : face_b;
+            const float proj = dot(delta, face);
+            const float err = len2(sub(delta, mul(face, proj)));
             if (err < best_err) {
                 best_err = err;
-                n = proj >= 0.0f ? faces[side] : mul(faces[side], -1.0f);
+                n = proj >= 0.0f ? face : mul(face, -1.0f);
             }
         }
     return n;
@@ -411,8 +444,8 @@ __device__ __noinline__ bool triangle_pair_contact(const RangeCtx& c, uint32_t a
     const V3 c_out_a = a_static && c.interior_a ? zero : out_a;
     const V3 c_out_b = b_static && c.interior_b ? zero : out_b;
     if (dot(out_a, out_b) > 0.9999f) return false;
-    V3 pa, pb;
-    closest_triangle_pair(A, B, pa, pb);
+    const ClosestPair near = closest_triangle_pair(A, B);
+    const V3 pa = near.a, pb = near.b;
     const V3 delta = sub(pa, pb);
     const float sq = len2(delta);
     if (sq > margin * margin) return false;
@@ -449,9 +482,8 @@ __device__ __noinline__ bool triangle_pair_contact(const RangeCtx& c, uint32_t a
     bool recovered = false;
     if (!am.solid && !bm.solid && dist <= 1.0e-5f) {
         const Tri oA = posed_tri(am, at, c.aprev), oB = posed_tri(bm, bt, c.bprev);
-        V3 opa, opb;
-        closest_triangle_pair(oA, oB, opa, opb);
-        V3 od = sub(opa, opb);
+        ClosestPair old = closest_triangle_pair(oA, oB);
+        V3 od = sub(old.a, old.b);
         if (len2(od) > 1.0e-10f) {
             Tri iA, iB;
             float low = 0.0f, high = 1.0f;
@@ -462,9 +494,8 @@ __device__ __noinline__ bool triangle_pair_contact(const RangeCtx& c, uint32_t a
                     iA.v[k] = add(oA.v[k], mul(sub(A.v[k], oA.v[k]), time));
                     iB.v[k] = add(oB.v[k], mul(sub(B.v[k], oB.v[k]), time));
                 }
-                V3 p, q;
-                closest_triangle_pair(iA, iB, p, q);
-                if (len2(sub(p, q)) > gap * gap)
+                const ClosestPair at_time = closest_triangle_pair(iA, iB);
+                if (len2(sub(at_time.a, at_time.b)) > gap * gap)
                     low = time;
                 else
                     high = time;
@@ -473,11 +504,11 @@ __device__ __noinline__ bool triangle_pair_contact(const RangeCtx& c, uint32_t a
                 iA.v[k] = add(oA.v[k], mul(sub(A.v[k], oA.v[k]), low));
                 iB.v[k] = add(oB.v[k], mul(sub(B.v[k], oB.v[k]), low));
             }
-            closest_triangle_pair(iA, iB, opa, opb);
-            od = sub(opa, opb);
-            c_n = triangle_feature_normal(iA, iB, opa, opb, normalized_or(od, fallback));
-            const V3 cpa = advect_triangle_point(opa, iA, A);
-            const V3 cpb = advect_triangle_point(opb, iB, B);
+            old = closest_triangle_pair(iA, iB);
+            od = sub(old.a, old.b);
+            c_n = triangle_feature_normal(iA, iB, old.a, old.b, normalized_or(od, fallback));
+            const V3 cpa = advect_triangle_point(old.a, iA, A);
+            const V3 cpb = advect_triangle_point(old.b, iB, B);
             c_p = mul(add(cpa, cpb), 0.5f);
             c_pen = rest - dot(sub(cpa, cpb), c_n) + 1.0e-5f;
             recovered = true;
@@ -538,15 +569,20 @@ __device__ __noinline__ bool triangle_pair_swept_contact(const RangeCtx& c, uint
     const V3 zero{0.0f, 0.0f, 0.0f};
     float time = 0.0f;
     bool starts_near = false, have_sep = false;
-    V3 sep_n = zero;
+    V3 sep_n = zero, last_pa = zero, last_pb = zero;
+    float last_time = 0.0f;
+    auto at_time = [&](float t, Tri& A, Tri& B) {
+#pragma unroll
+        for (uint32_t k = 0; k < 3; ++k) {
+            A.v[k] = add(PA.v[k], mul(DA.v[k], t));
+            B.v[k] = add(PB.v[k], mul(DB.v[k], t));
+        }
+    };
     for (uint32_t it = 0; it < 32; ++it) {
         Tri A, B;
-        for (uint32_t k = 0; k < 3; ++k) {
-            A.v[k] = add(PA.v[k], mul(DA.v[k], time));
-            B.v[k] = add(PB.v[k], mul(DB.v[k], time));
-        }
-        V3 pa, pb;
-        closest_triangle_pair(A, B, pa, pb);
+        at_time(time, A, B);
+        const ClosestPair near = closest_triangle_pair(A, B);
+        const V3 pa = near.a, pb = near.b;
         const V3 delta = sub(pa, pb);
         const float dist = sqrtf(fmx(0.0f, len2(delta)));
         float offset = rest;
@@ -581,6 +617,14 @@ __device__ __noinline__ bool triangle_pair_swept_contact(const RangeCtx& c, uint
                 fallback = c_out_b;
             else if (len2(c_out_a) > 0.5f)
                 fallback = mul(c_out_a, -1.0f);
+            if (have_sep && !c.guided) {
+                // The last separated step's feature normal, formed only now
+                // that it is used.
+                Tri LA, LB;
+                at_time(last_time, LA, LB);
+                sep_n = triangle_feature_normal(LA, LB, last_pa, last_pb,
+                                                normalized_or(sub(last_pa, last_pb), V3{0.0f, 1.0f, 0.0f}));
+            }
             const V3 nrm = triangle_feature_normal(A, B, pa, pb, have_sep ? sep_n : fallback);
             if (!shell_contact_facing(nrm, c_out_a, c_out_b)) return false;
             const V3 point = mul(add(pa, pb), 0.5f);
@@ -593,10 +637,13 @@ __device__ __noinline__ bool triangle_pair_swept_contact(const RangeCtx& c, uint
             c_impact = starts_near ? 0.0f : time;
             return true;
         }
-        sep_n = triangle_feature_normal(A, B, pa, pb, normalized_or(delta, V3{0.0f, 1.0f, 0.0f}));
+        last_time = time;
+        last_pa = pa;
+        last_pb = pb;
         have_sep = true;
         float adv = (dist - offset) / (bound + kEps) * 0.9f;
         if (c.guided) {
+            sep_n = triangle_feature_normal(A, B, pa, pb, normalized_or(delta, V3{0.0f, 1.0f, 0.0f}));
             // Advance by the gap along the separating feature plane when that
             // is faster; a separating, opening gap ends the search.
             const V3 plane = triangle_feature_normal(A, B, pa, pb, sep_n);
