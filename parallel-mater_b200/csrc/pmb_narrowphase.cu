@@ -725,10 +725,13 @@ __device__ __noinline__ void narrow_outgrown(const Dev& d, uint32_t k, uint2 sat
 
 // Pass 2, a thread or 16 lanes per surviving candidate. With few survivors
 // the serial chain is what counts (217: 43 us with lanes, 124 with threads);
-// with many, the lanes' extra work (25,000: 176 and 190 us; 412,000: 2.36 and
-// 0.97 ms). The survivors' number is not known at the launch; piles have
-// about six a body, so worlds of up to kLaneBodies bodies take the lanes.
-constexpr uint32_t kLaneBodies = 3072;
+// with many, the lanes' extra work (412,000: 2.36 and 0.97 ms). The survivors'
+// number is not known at the launch; piles have about six a body, so worlds of
+// up to kLaneBodies bodies take the lanes (4,096 boxes, 25,000 survivors: a
+// tick of 1,540 us against 1,658). The threads' polygons in shared memory
+// instead of local memory were slower (1.91 ms against 0.97 at 412,000): a
+// third fewer threads fit, and a warp waits for its longest polygon either way.
+constexpr uint32_t kLaneBodies = 6144;
 __global__ void __launch_bounds__(128, 6) k_narrow(Dev d) {
     tick_begin();
     const uint32_t total = d.ctr->n_surv;
