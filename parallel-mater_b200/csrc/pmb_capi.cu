@@ -356,7 +356,7 @@ int allocate_world(pmb_world* w, Dev& d, const Sizes& z, Extra& e) {
     ALLOC(d.lo, n); ALLOC(d.hi, n); ALLOC(d.is_large, n); ALLOC(d.large_list, n);
     ALLOC(d.bucket_count, grid_size + 1); ALLOC(d.bucket_off, grid_size + 1); ALLOC(d.bucket_cursor, grid_size);
     ALLOC(d.grid_body, n); ALLOC(d.grid_cell, n);
-    ALLOC(d.cand_count, n + 1); ALLOC(d.cand_off, n + 1); ALLOC(d.cand_lane, kQueryLanes * size_t(n));
+    ALLOC(d.cand_count, n + 1); ALLOC(d.cand_off, n + 1); ALLOC(d.cand_kept, kQueryKept * size_t(n));
     ALLOC(d.cand_a, cap_cand); ALLOC(d.cand_b, cap_cand);
     ALLOC(d.np_count, cap_cand); ALLOC(d.np_scan, cap_cand + 1); ALLOC(d.np_stage, cap_cand);
     ALLOC(d.np_list, cap_cand); ALLOC(d.np_sat, cap_cand);

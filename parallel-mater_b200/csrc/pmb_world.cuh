@@ -24,6 +24,7 @@ enum : uint32_t { kStatic = 0, kKinematic = 1, kDynamic = 2 };
 enum : uint32_t { kFixed, kPoint, kHinge, kSlider, kPiston, kGeneric, kGenericSpring, kMotor };
 constexpr uint32_t kMaxColors = 256;
 constexpr uint32_t kQueryLanes = 8;  // broadphase query lanes per body
+constexpr uint32_t kQueryKept = 64;  // candidates of a body kept for the write pass
 // The colour fixpoint runs one 1024-thread CTA per SM: its ~30 rounds are
 // two grid barriers each, and a barrier's cost grows with the CTA count.
 constexpr int kColorThreads = 1024;
@@ -226,7 +227,7 @@ struct Dev {
     uint32_t* grid_body;
     int4* grid_cell;
     uint32_t *cand_count, *cand_off;
-    uint32_t* cand_lane;  // per query body, each query lane's candidate count
+    uint32_t* cand_kept;  // per query body, its first kQueryKept candidates
     uint32_t *cand_a, *cand_b;
     // narrowphase
     uint32_t* np_count;
