@@ -455,14 +455,13 @@ __device__ __forceinline__ void mark_higher(const Dev& d, uint32_t v, uint8_t* n
 __global__ void __launch_bounds__(kColorThreads) k_color(Dev d) {
     Counters* c = d.ctr;
     if (c->status & kStBarrierTimeout) return;  // the tick was abandoned
-    // The change counter is read by one thread per block and shared: a read
-    // by every thread of the grid per round piles onto one L2 line.
-    __shared__ uint32_t s_before, s_after;
+    // A round's changes go to one of three counters: read by one thread per
+    // block after the round's barrier (a read by every thread of the grid
+    // piles onto one L2 line) and cleared two rounds later, when every block
+    // is past reading it. So a round needs one barrier.
+    __shared__ uint32_t s_changed;
     uint32_t arrivals = 0;  // grid_sync
     for (uint32_t round = 0; round < d.n + 2; ++round) {
-        if (threadIdx.x == 0) s_before = ((volatile uint32_t*)&c->changed)[0];
-        if (!grid_sync(c, kBarColor, arrivals, d.barrier_spins)) return;
-        const uint32_t before = s_before;
         uint8_t* cur = d.cdirty + size_t(round & 1u) * d.n;
         uint8_t* next = d.cdirty + size_t((round + 1u) & 1u) * d.n;
         bool transient = false;  // a mex past 255 in this round (judged at the fixpoint)
@@ -481,12 +480,14 @@ __global__ void __launch_bounds__(kColorThreads) k_color(Dev d) {
             }
         }
         changes = __reduce_add_sync(0xffffffffu, changes);  // one atomic per warp
-        if (changes && (threadIdx.x & 31) == 0) atomicAdd(&c->changed, changes);
+        if (changes && (threadIdx.x & 31) == 0) atomicAdd(&c->changed[round % 3u], changes);
+        if (grid_stride_begin() == 0) c->changed[(round + 1u) % 3u] = 0;
         if (!grid_sync(c, kBarColor, arrivals, d.barrier_spins)) return;
-        if (threadIdx.x == 0) s_after = ((volatile uint32_t*)&c->changed)[0];
+        if (threadIdx.x == 0) s_changed = ((volatile uint32_t*)c->changed)[round % 3u];
         __syncthreads();
-        const uint32_t after = s_after;
-        if (after == before) {
+        const bool settled = s_changed == 0;
+        __syncthreads();  // (read before the next round's write)
+        if (settled) {
             // Converged. A body's mex can pass 255 colours in an intermediate
             // round and still settle below 256, so overflow is judged on the
             // final colours: a body left at the last colour whose lower

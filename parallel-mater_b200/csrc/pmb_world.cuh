@@ -59,7 +59,7 @@ enum : uint32_t {
 struct Counters {
     uint32_t n_cand, n_stage, n_act, n_contacts;
     uint32_t n_large, colors, islands, iterations;
-    uint32_t impact, status, changed, rounds;
+    uint32_t impact, status, changed[3], rounds;
     uint32_t bar[3], budget, joint_iters;
     float hs, residual, pad1, pad2;
     uint32_t budget_max;  // batched scenes: the largest scene budget of the tick
