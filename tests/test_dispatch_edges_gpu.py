@@ -1,0 +1,111 @@
+# SPDX-License-Identifier: MIT
+"""The tick's size-dependent branches at their edges, against the oracle.
+
+A tick picks kernels and grids by the world's size: one solve block up to 40
+bodies, narrowphase lanes up to 6,144, one-block grid and colour order up to
+8,192; a query keeps 64 candidates; a lane group takes two, five or ten joints
+of a body at a time. Every branch evaluates the serial order's operations, so states,
+candidate pairs and colours are compared bit for bit.
+"""
+import numpy as np
+import pytest
+
+import oracle as O
+from pmb200 import core, scenes
+
+pytestmark = pytest.mark.gpu
+
+
+def _same(scene, ticks, **kw):
+    w, o = core.World(scene), O.OracleWorld(scene)
+    contacts = 0
+    for t in range(ticks):
+        sg, so = w.step(**kw), o.step(**kw)
+        assert sg["status"] == 0, core.status_names(int(sg["status"]))
+        for k in ("candidate_pairs", "active_pairs", "contacts", "colors", "islands"):
+            assert sg[k] == so[k], (t, k)
+        assert np.array_equal(w.candidate_pairs(), o.candidate_pairs()), t
+        dyn = scene.bodies["motion"] == scenes.DYNAMIC
+        assert np.array_equal(w.graph()[0][dyn], o.graph()[0][dyn]), t
+        assert np.array_equal(w.states().view(np.uint8), o.states().view(np.uint8)), t
+        contacts = max(contacts, int(sg["contacts"]))
+    w.close()
+    return contacts
+
+
+# box_pile adds five static bodies; boxes 1.4 m apart touch from the start.
+@pytest.mark.parametrize("bodies", [6, 40, 41, 130, 1030, 6144, 6145, 8192, 8193])
+def test_world_sizes_around_the_dispatch_edges(gpu_available, bodies):
+    side = max(1, int(np.ceil((bodies - 5) ** (1.0 / 3.0))))
+    scene = scenes.box_pile((side, side, side), seed=bodies, spacing=1.4, count=bodies - 5)
+    assert scene.n == bodies
+    assert _same(scene, 6 if bodies < 2000 else 2) > 0 or bodies < 10
+
+
+def test_query_with_more_candidates_than_are_kept(gpu_available):
+    """A plate over 12 x 12 boxes (144 candidates) and boxes below the kept
+    number, in one world."""
+    b = scenes._Builder()
+    scenes._ground(b, 20.0, 20.0)
+    cube = b.mesh(*scenes.box_mesh((0.25, 0.25, 0.25)))
+    plate = b.mesh(*scenes.box_mesh((4.0, 0.1, 4.0)))
+    b.body(plate, scenes.DYNAMIC, (0.0, 0.62, 0.0), mass=5.0, inertia=scenes.box_inertia(5.0, (4.0, 0.1, 4.0)))
+    for k in range(144):
+        x, z = (k % 12 - 5.5) * 0.6, (k // 12 - 5.5) * 0.6
+        b.body(cube, scenes.DYNAMIC, (x, 0.2505, z), mass=1.0, inertia=scenes.box_inertia(1.0, (0.25,) * 3))
+    assert _same(b.build("plate", 10), 4) > 0
+
+
+@pytest.mark.parametrize("joints", [1, 2, 3, 5, 6, 11, 23])
+def test_bodies_with_many_joints(gpu_available, joints):
+    """A hub joined to `joints` boxes by joints of every type in turn (generic
+    and spring joints have more rows an axis than a lane's slot holds)."""
+    b = scenes._Builder()
+    hub = b.mesh(*scenes.box_mesh((0.3, 0.3, 0.3)))
+    small = b.mesh(*scenes.box_mesh((0.05, 0.05, 0.05)))
+    h = b.body(hub, scenes.DYNAMIC, (0.0, 3.0, 0.0), w=(0.3, 0.5, -0.2), mass=4.0,
+               inertia=scenes.box_inertia(4.0, (0.3,) * 3))
+    rng = np.random.Generator(np.random.Philox(joints))
+    for k in range(joints):
+        a = 2.0 * np.pi * k / joints
+        x = np.array([np.cos(a), 0.2 * (k % 3), np.sin(a)])
+        v = tuple(float(q) for q in rng.uniform(-1, 1, 3))
+        i = b.body(small, scenes.DYNAMIC, tuple(float(q) for q in x + (0.0, 3.0, 0.0)), v=v, mass=0.5,
+                   inertia=scenes.box_inertia(0.5, (0.05,) * 3))
+        j = b.joint(k % 8, h, i, tuple(float(q) for q in 0.5 * x), tuple(float(q) for q in -0.5 * x))
+        o = b.joints[j]
+        o["lin_limit_axes"] = o["ang_limit_axes"] = 7
+        o["lin_lower"], o["lin_upper"] = (-0.1, -0.1, 0.0), (0.2, 0.1, 0.0)
+        o["ang_lower"], o["ang_upper"] = (-0.3, -0.2, -0.4), (0.3, 0.2, 0.4)
+        o["lin_spring_axes"] = o["ang_spring_axes"] = 7
+        o["lin_stiffness"], o["lin_damping"] = (200.0,) * 3, (5.0,) * 3
+        o["ang_stiffness"], o["ang_damping"] = (50.0,) * 3, (1.0,) * 3
+        o["motor_angular"] = o["motor_linear"] = 1
+        o["motor_angular_velocity"], o["motor_angular_max_impulse"] = 2.0, 5.0
+        o["motor_linear_velocity"], o["motor_linear_max_impulse"] = 0.5, 3.0
+    _same(b.build("hub", 12), 12)
+
+
+def test_block_solves_over_forty_decades(gpu_available):
+    """Random symmetric positive blocks, with zero entries and entries near
+    the ends of the 32-bit range: the device's solution is the serial one's
+    bit pattern."""
+    rng = np.random.Generator(np.random.Philox(12))
+    rows = []
+    for k in range(20000):
+        m = rng.uniform(-1, 1, (6, 6)) * 10.0 ** rng.uniform(-3, 3, (6, 1))
+        h = m @ m.T + np.diag(10.0 ** rng.uniform(-4, 2, 6))
+        if k % 3 == 0:
+            h[3:, :3] = h[:3, 3:] = 0.0
+        h = h * 10.0 ** rng.uniform(-20, 15)
+        g = rng.uniform(-1, 1, 6) * 10.0 ** rng.uniform(-22, 12)
+        if k % 5 == 0:
+            g[rng.integers(0, 6, 3)] = -0.0
+        rows.append(np.concatenate([[h[r, c] for r in range(6) for c in range(r + 1)], g]))
+    x = np.array(rows, np.float32)
+    out = core.math_eval(0, x)
+    want = [O.block_solve(r[:21], r[21:]) for r in x]
+    assert np.array_equal(out[:, 6].astype(bool), np.array([bool(w[0]) for w in want]))
+    got, ref = out[:, :6].copy(), np.array([w[1] for w in want], np.float32)
+    assert np.array_equal(got.view(np.uint32), ref.view(np.uint32))
+    assert (out[:, 6] == 1).sum() > 15000
