@@ -1116,10 +1116,11 @@ struct SweepResidual {
     bool met;
 };
 // Every block needs the same decision, so every block sums the partials in
-// slot order. One warp per block reads them -- each lane a slot of every 32,
-// all loads in flight at once -- and the block shares the result: when every
-// thread walked the slots itself, the whole grid's uncached reads of the same
-// few L2 lines kept each sweep's start waiting tens of microseconds.
+// the same order. One warp per block reads them -- each lane the slots of its
+// index modulo 32, all loads in flight at once -- and adds the lanes' sums in
+// a tree (when every thread walked the slots itself, the whole grid's
+// uncached reads of the same few L2 lines kept each sweep's start waiting
+// tens of microseconds; the 148 slots one after another took 2 us a sweep).
 __device__ __forceinline__ SweepResidual sweep_residual(Counters* c, uint32_t base, const StepParams& sp) {
     __shared__ SweepResidual shared_result;
     if (threadIdx.x < 32) {
@@ -1141,18 +1142,18 @@ __device__ __forceinline__ SweepResidual sweep_residual(Counters* c, uint32_t ba
                 mx[j] = in ? ((volatile float*)c->res_mx)[base + k] : 0.0f;
                 ov[j] = in ? ((volatile uint32_t*)c->res_over)[base + k] : 0u;
             }
-            // Slot order: chunk j, then lanes in order (the same additions
-            // as a serial walk over the slots).
 #pragma unroll
-            for (uint32_t j = 0; j < kAhead; ++j)
-                for (uint32_t l = 0; l < 32u; ++l) {
-                    if (k0 + 32u * j + l >= gridDim.x) break;
-                    tsq += __shfl_sync(0xffffffffu, sq[j], int(l));
-                    tn += __shfl_sync(0xffffffffu, cn[j], int(l));
-                    tmx = fmx(tmx, __shfl_sync(0xffffffffu, mx[j], int(l)));
-                    to += __shfl_sync(0xffffffffu, ov[j], int(l));
-                }
+            for (uint32_t j = 0; j < kAhead; ++j) {
+                tsq += sq[j];
+                tn += cn[j];
+                tmx = fmx(tmx, mx[j]);
+                to += ov[j];
+            }
         }
+        for (int o = 16; o > 0; o >>= 1) tsq += __shfl_xor_sync(0xffffffffu, tsq, o);
+        for (int o = 16; o > 0; o >>= 1) tmx = fmx(tmx, __shfl_xor_sync(0xffffffffu, tmx, o));
+        tn = __reduce_add_sync(0xffffffffu, tn);
+        to = __reduce_add_sync(0xffffffffu, to);
         if (lane == 0) {
             SweepResidual r;
             r.rms = tn ? float(sqrt(tsq / double(tn))) : 0.0f;

@@ -109,3 +109,22 @@ def test_block_solves_over_forty_decades(gpu_available):
     got, ref = out[:, :6].copy(), np.array([w[1] for w in want], np.float32)
     assert np.array_equal(got.view(np.uint32), ref.view(np.uint32))
     assert (out[:, 6] == 1).sum() > 15000
+
+
+def test_a_body_per_thread(gpu_available):
+    """Colours with more bodies than a round of 16-lane groups holds give them
+    a thread each (policy 4): 21,952 boxes, contacts from the start, the same
+    bits as the oracle under every CTA size."""
+    scene = scenes.box_pile((28, 28, 28), seed=3, spacing=1.42)
+    o = O.OracleWorld(scene)
+    want = []
+    for _ in range(2):
+        o.step(iterations=3)
+        want.append(o.states().view(np.uint8).copy())
+    for variant in (0, 1, 2):
+        w = core.World(scene)
+        w.set_launch_plan(variant, 4)
+        for t in range(2):
+            assert w.step(iterations=3)["status"] == 0
+            assert np.array_equal(w.states().view(np.uint8), want[t]), (variant, t)
+        w.close()
