@@ -426,7 +426,8 @@ PMB_API int pmb_world_scene_stats(pmb_world* world, float* residual, float* resi
  * cover the whole colour, 3 = widths as 0 with the colour's bodies claimed
  * dynamically from a counter, 4 = one thread per body in colours with more
  * bodies than 16-lane groups, else as 0. Every plan computes bit-identical
- * results; only the speed differs. A new world starts with (0, 0). */
+ * results; only the speed differs. A new world starts with policy 0 and the
+ * variant its body and joint counts suggest. */
 PMB_API int pmb_world_set_launch_plan(pmb_world* world, uint32_t solve_variant, uint32_t solve_policy);
 /* Bound on the polls a thread block makes at a grid barrier of the tick's
  * cooperative kernels (colouring fixpoint, solve) before it gives up (0: the

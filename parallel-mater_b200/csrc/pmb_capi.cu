@@ -171,6 +171,21 @@ __global__ void k_reset_counters(Dev d) {
         }
 }
 
+// The CTA size a world starts with (pmb_world_autotune measures its own).
+// Fewer threads leave each more registers (no spills, more of a chain in
+// flight) where a colour does not fill the grid anyway: 256 threads up to
+// 3,072 bodies, and up to 16,384 with joints, whose rows take the most
+// registers (us a tick with 512, 384, 256 threads: 56 bodies 457, 446, 430;
+// joint rigs, 224: 763, 729, 710; 2,202 boxes 1,180, 1,174, 1,137; 128 chains,
+// 8,448: 3,032, 2,926, 2,806). Beyond, 512 fill it (4,101 boxes 1,468, 1,498,
+// 1,473; 512 chains, 33,792: 4,584, 4,939, 5,350), but for the largest joint-
+// free worlds, many rounds a colour, 384 (65,541 boxes to a residual 24.1,
+// 23.6, 24.9 ms; 8 sweeps 5,020, 5,027, 5,195).
+uint32_t starting_variant(uint32_t bodies, uint32_t joints) {
+    if (bodies <= (joints ? 16384u : 3072u)) return 2;
+    return !joints && bodies > 32768u ? 1 : 0;
+}
+
 // Blocks of the cooperative kernels. Few bodies need few blocks: a barrier
 // costs more the more blocks arrive (1.1 us of 148, 0.5 of 8), and one block
 // needs none and keeps the world in its L1. Colouring: a block of
@@ -721,7 +736,7 @@ int pmb_world_create(const pmb_world_desc* desc, pmb_world** out) {
     std::vector<float> sorted = expand;
     std::nth_element(sorted.begin(), sorted.begin() + n / 2, sorted.end());
     d.large_extent = 2.0f * sorted[n / 2] * 4.0f;
-    d.solve_variant = 0;  // 512 threads: the fastest plan on a settled 65k-box pile
+    d.solve_variant = starting_variant(n, nj);
     d.solve_policy = 0;
     d.barrier_spins = kDefaultBarrierSpins;
     for (uint32_t v = 0; v < kSolveVariants; ++v) {
