@@ -431,7 +431,7 @@ PMB_API int pmb_world_scene_stats(pmb_world* world, float* residual, float* resi
 PMB_API int pmb_world_set_launch_plan(pmb_world* world, uint32_t solve_variant, uint32_t solve_policy);
 /* Bound on the polls a thread block makes at a grid barrier of the tick's
  * cooperative kernels (colouring fixpoint, solve) before it gives up (0: the
- * default, 2^26 polls, seconds). A barrier that runs out latches
+ * default, 2^26 polls, tens of seconds). A barrier that runs out latches
  * PMB_STATUS_BARRIER_TIMEOUT in the tick's status, the remaining cooperative
  * kernels of the tick return at once and the host reads the status after the
  * tick (the pm* driver reports it as PM_ERROR_DEVICE_LOST); the next tick

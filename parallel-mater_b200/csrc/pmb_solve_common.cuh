@@ -880,7 +880,7 @@ __device__ __forceinline__ void res_add(Res& r, float v) {
 }
 
 // advance_duals for one contact point (geometry_constraints_solve.slang:
-// 494-532; the last-iteration block runs in k_contact_finalize). ab: the
+// 494-532; the last-iteration block runs in k_finish_contacts). ab: the
 // contact's bodies (c_bodies[c]), loaded by the caller ahead of time.
 static __device__ void dual_contact(const Dev& d, uint32_t c, uint2 ab, float dt, uint32_t phase, Res& res,
                                     uint32_t it) {

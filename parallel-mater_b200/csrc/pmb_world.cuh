@@ -270,7 +270,7 @@ struct Dev {
     uint32_t* corder;
     uint4* crec;  // per colour-order slot: body, row offset, row count, impact flag (the solve's body records)
     uint8_t* cdirty;  // colour rounds: two flag arrays of n (bodies to revisit)
-    uint32_t *nbr, *nlow, *nhigh;  // dynamic neighbours per body (k_neighbour_lists)
+    uint32_t *nbr, *nlow, *nhigh;  // dynamic neighbours per body (k_graph_rows)
     ContactEvent* events;
     uint32_t event_capacity;
     uint32_t *rcount, *roff, *blist;  // per-body flattened contact rows (bit 31: second body)
