@@ -664,6 +664,9 @@ __device__ void solve_body_group(const Dev& d, Ahead& ah, uint32_t kn, uint32_t 
         __syncwarp(gmask);
         Blk blk;
         read_block<G>(sm, blk);
+        // Every lane has read the block before a lane writes its words again:
+        // the second pass's entries, or the next body's rows.
+        __syncwarp(gmask);
         V6 x;
         const bool solved = block_solve(blk, x);
         if (pass != 0) {

@@ -128,3 +128,35 @@ def test_a_body_per_thread(gpu_available):
             assert w.step(iterations=3)["status"] == 0
             assert np.array_equal(w.states().view(np.uint8), want[t]), (variant, t)
         w.close()
+
+
+def test_groups_that_solve_resting_and_flying_bodies_in_turn(gpu_available):
+    """A lane group's next body reuses the shared memory its lanes read the
+    last one's block from. 12,544 boxes of one colour, half of them in the air
+    (no rows: the block is the first thing written) and the others sliding or
+    lifting off (crossing rows, two passes), mixed in one sort class: more than
+    a round for the groups of every CTA size."""
+    b = scenes._Builder()
+    side = 112
+    scenes._ground(b, 1.5 * side + 5.0, 1.5 * side + 5.0)
+    cube = b.mesh(*scenes.box_mesh((0.5, 0.5, 0.5)))
+    rng = np.random.Generator(np.random.Philox(8))
+    for k in range(side * side):
+        x, z = (k % side - 0.5 * side) * 3.0, (k // side - 0.5 * side) * 3.0
+        v = rng.uniform(-1, 1, (2, 3))
+        b.body(cube, scenes.DYNAMIC, (x, 0.499 if rng.random() < 0.5 else 5.0, z), v=tuple(map(float, v[0])),
+               w=tuple(map(float, v[1])), mass=1.0, inertia=scenes.box_inertia(1.0, (0.5,) * 3))
+    scene = b.build("resting and flying", 4)
+    o = O.OracleWorld(scene)
+    want = []
+    for _ in range(3):
+        o.step()
+        want.append(o.states().view(np.uint8).copy())
+    for variant in (0, 1, 2):
+        w = core.World(scene)
+        w.set_launch_plan(variant, 1)
+        for t in range(3):
+            st = w.step()
+            assert st["status"] == 0 and st["colors"] == 1 and st["contacts"] > 10000
+            assert np.array_equal(w.states().view(np.uint8), want[t]), (variant, t)
+        w.close()
