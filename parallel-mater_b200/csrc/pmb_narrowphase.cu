@@ -518,6 +518,7 @@ __device__ __forceinline__ void reduce_patch_lanes(const LaneGroup& g, LaneMan& 
 __device__ __forceinline__ bool face_manifold_lanes(const LaneGroup& g, const Pose& bs, const MeshRef& bm,
                                                     const Pose& cs, const MeshRef& cm, float margin, float correction,
                                                     LaneMan& out, const FaceSat& fs, ClipShared& sm, bool& outgrown) {
+    __syncwarp(g.mask);  // an earlier manifold's last polygon is read
     out.count = 0;
     out.normal = out.p = {0, 0, 0};
     out.pen = 0.0f;

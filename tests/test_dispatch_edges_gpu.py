@@ -160,3 +160,24 @@ def test_groups_that_solve_resting_and_flying_bodies_in_turn(gpu_available):
             assert st["status"] == 0 and st["colors"] == 1 and st["contacts"] > 10000
             assert np.array_equal(w.states().view(np.uint8), want[t]), (variant, t)
         w.close()
+
+
+def test_translating_pairs_that_try_several_manifolds(gpu_available):
+    """Boxes that move more than their margin without turning: sliding ones
+    touch at the start (the predicted poses), rising ones no longer do (the
+    start's poses, then the correction's), falling ones touch on the way --
+    the polygons of one pair's manifolds share the lanes' shared memory."""
+    b = scenes._Builder()
+    scenes._ground(b, 60.0, 60.0)
+    cube = b.mesh(*scenes.box_mesh((0.5, 0.5, 0.5)))
+    rng = np.random.Generator(np.random.Philox(21))
+    for k in range(96):
+        x, z = (k % 12 - 5.5) * 2.0, (k // 12 - 3.5) * 2.0
+        kind = k % 4
+        y, v = [(0.5005, (6.0, 0.0, 2.0)), (0.5005, (0.5, 6.0, 0.0)), (1.1, (3.0, -40.0, 1.0)),
+                (1.1, (60.0, -20.0, 45.0))][kind]
+        v = tuple(float(q) for q in np.array(v) * rng.uniform(0.7, 1.3))
+        for up in range(2):
+            b.body(cube, scenes.DYNAMIC, (x + 0.1 * up, y + 1.0005 * up, z), v=v, mass=1.0,
+                   inertia=scenes.box_inertia(1.0, (0.5,) * 3))
+    assert _same(b.build("translating", 8), 4) > 0
