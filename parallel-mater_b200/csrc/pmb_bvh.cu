@@ -218,11 +218,9 @@ __global__ void k_bvh_top_bounds(uint32_t n, uint32_t level, const uint32_t* lis
     const uint32_t first = warp * kBoundsPerWarp;
     uint32_t held = kInvalid;
     uint32_t k[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
-    auto flush = [&] {
+    auto flush = [&] {  // by the whole warp
         uint32_t* a = acc + 6 * size_t(held);
-        const uint32_t same = __match_any_sync(__activemask(), held);
-        const uint32_t all = __activemask();
-        if (same == all && all == 0xffffffffu) {
+        if (__match_any_sync(0xffffffffu, held) == 0xffffffffu) {
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
                 k[c] = __reduce_min_sync(0xffffffffu, k[c]);
