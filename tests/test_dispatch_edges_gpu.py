@@ -16,8 +16,8 @@ from pmb200 import core, scenes
 pytestmark = pytest.mark.gpu
 
 
-def _same(scene, ticks, **kw):
-    w, o = core.World(scene), O.OracleWorld(scene)
+def _same(scene, ticks, contact_capacity=0, **kw):
+    w, o = core.World(scene, contact_capacity=contact_capacity), O.OracleWorld(scene)
     contacts = 0
     for t in range(ticks):
         sg, so = w.step(**kw), o.step(**kw)
@@ -180,4 +180,6 @@ def test_translating_pairs_that_try_several_manifolds(gpu_available):
         for up in range(2):
             b.body(cube, scenes.DYNAMIC, (x + 0.1 * up, y + 1.0005 * up, z), v=v, mass=1.0,
                    inertia=scenes.box_inertia(1.0, (0.5,) * 3))
-    assert _same(b.build("translating", 8), 4) > 0
+    # Pairs without a face manifold take the triangle path: at most 2 x 12 x 12
+    # triangle pairs for each of at most 1,600 candidates.
+    assert _same(b.build("translating", 8), 4, contact_capacity=1600 * 288) > 0
