@@ -44,6 +44,7 @@ __device__ __forceinline__ void prepare_bodies(const Dev& d, const StepParams& s
         d.jdeg[i] = 0;
         d.inc_cursor[i] = 0;
         d.jinc_cursor[i] = 0;
+        if (!d.nj) d.jinc_off[i] = 0;  // (with joints the scan of jdeg writes them)
         d.cdirty[i] = d.cdirty[size_t(d.n) + i] = 0;
         if (d.motion[i] != kDynamic) {
             d.color[i] = kInvalid;
@@ -618,8 +619,8 @@ void launch_graph(const Dev& d, const StepParams& sp, cudaStream_t s, int coop_b
     uint32_t gb = cap_blocks(d.cap_pair > d.nj ? d.cap_pair : d.nj);
     const uint32_t db = cap_blocks(std::max({d.cap_pair, d.nj, d.cap_contact}));
     launch(k_graph_degrees, db, kBlock, s, d, sp);
-    // (Without joints the joint lists' offsets stay the zeros of the world's
-    // creation.)
+    // (Without joints prepare_bodies zeroes the joint lists' offsets: scratch
+    // memory may be the caller's, who may write it between ticks.)
     if (d.nj)
         scan_u32_pair(d.deg, d.inc_off, nullptr, d.jdeg, d.jinc_off, nullptr, nullptr, d.n, d.scan_tmp32, s);
     else
