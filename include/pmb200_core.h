@@ -311,8 +311,9 @@ PMB_API int pmb_world_copy_states_to_device(pmb_world* world, uint32_t first, ui
  * (realtime_telemetry.hpp: boundary, predict, index, candidates, domain,
  * coupling, commit): kernel dispatches and thread blocks enqueued per phase,
  * algorithmic bytes per phase (the per-body and per-contact costs of the
- * kernels), grid-wide barriers (colour rounds and sweeps), sweeps and
- * spatial-index builds. Feeds PM_QUERY_REALTIME_STEP_STATISTICS. */
+ * kernels), grid-wide barriers (one per colour round; per sweep one per colour
+ * and, unless the launch plan fuses them, one after the duals; a grid of one
+ * block passes them with its own barrier), sweeps and spatial-index builds. Feeds PM_QUERY_REALTIME_STEP_STATISTICS. */
 typedef struct pmb_tick_telemetry {
     uint64_t tick;
     uint64_t dispatches[7], workgroups[7], bytes_moved[7], barriers[7];

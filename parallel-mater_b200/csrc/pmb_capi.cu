@@ -1218,7 +1218,13 @@ int pmb_world_tick_telemetry(pmb_world* w, pmb_tick_telemetry* out) {
     const uint64_t sweeps = uint64_t(c.iterations) + (c.impact ? uint64_t(c.budget) : 0u);
     out->sweeps = sweeps;
     out->spatial_builds = 1;
-    out->barriers[kPhDomain] = 2ull * c.rounds + sweeps * (uint64_t(c.colors) + 1u);
+    // One barrier a colour round; in a sweep one a colour and one after the
+    // duals, which the staged solve does with the last colour. (Without colours
+    // a sweep waits twice, the last once.) A grid of one block passes the same
+    // points with its own barrier.
+    const bool staged = w->d.solve_variant >= kStagedFirst;
+    out->barriers[kPhDomain] = c.rounds + (c.colors ? sweeps * (uint64_t(c.colors) + (staged ? 0u : 1u))
+                                                    : staged || sweeps == 0 ? sweeps : 2u * sweeps - 1u);
     out->bytes_moved[kPhPredict] = 250u * n;
     out->bytes_moved[kPhIndex] = 100u * n;
     out->bytes_moved[kPhCandidates] = 8ull * c.n_cand + 64u * con;

@@ -7,6 +7,9 @@ bodies, narrowphase lanes up to 6,144, one-block grid and colour order up to
 of a body at a time. Every branch evaluates the serial order's operations, so states,
 candidate pairs and colours are compared bit for bit.
 """
+import ctypes
+import re
+
 import numpy as np
 import pytest
 
@@ -183,3 +186,36 @@ def test_translating_pairs_that_try_several_manifolds(gpu_available):
     # Pairs without a face manifold take the triangle path: at most 2 x 12 x 12
     # triangle pairs for each of at most 1,600 candidates.
     assert _same(b.build("translating", 8), 4, contact_capacity=1600 * 288) > 0
+
+
+class _Telemetry(ctypes.Structure):
+    _fields_ = [("tick", ctypes.c_uint64)] + [(k, ctypes.c_uint64 * 7) for k in
+                                              ("dispatches", "workgroups", "bytes_moved", "barriers")] + \
+               [("sweeps", ctypes.c_uint64), ("spatial_builds", ctypes.c_uint64)]
+
+
+def _telemetry(w):
+    t = _Telemetry()
+    f = core.lib().pmb_world_tick_telemetry
+    f.argtypes = [ctypes.c_void_p, ctypes.c_void_p]
+    assert f(w.h, ctypes.byref(t)) == 0
+    return t
+
+
+@pytest.mark.parametrize("variant", [0, 3])
+@pytest.mark.parametrize("boxes", [20, 2000])
+def test_telemetry_counts_the_barriers_a_tick_passes(gpu_available, boxes, variant):
+    """One barrier a colour round; in a sweep one a colour and, in the group
+    variants, one after the duals. A legacy tick with an impact sweeps twice."""
+    w = core.World(scenes.box_pile((13, 13, 13), seed=5, spacing=1.4, count=boxes))
+    w.set_launch_plan(variant, 0)
+    for _ in range(4):
+        w.step(stats=False)
+    report = w.profile_step()
+    st, t = w.stats(), _telemetry(w)
+    rounds = int(re.search(r"rounds (\d+)", report).group(1))
+    sweeps = int(st["iterations"]) * (2 if st["impact"] else 1)
+    assert rounds >= 1 and st["colors"] > 1 and t.sweeps == sweeps > 0
+    assert t.barriers[4] == rounds + sweeps * (int(st["colors"]) + (1 if variant < 3 else 0))
+    assert sum(t.barriers) == t.barriers[4]
+    w.close()
