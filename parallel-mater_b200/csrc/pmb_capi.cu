@@ -87,6 +87,7 @@ struct pmb_world {
     Counters host_ctr{};
     LaunchLedger ledger{};          // launches of the latest enqueued tick
     uint64_t ticks_enqueued{};
+    uint32_t solve_phases{};        // of the latest enqueued tick: realtime ticks have no velocity phase
     // Learned warm start (allocated by pmb_world_mlp_attach).
     struct Mlp {
         bool attached{}, train{};
@@ -257,6 +258,7 @@ void enqueue_step(pmb_world* w, const StepParams& sp) {
     }
     g_ledger = nullptr;
     ++w->ticks_enqueued;
+    w->solve_phases = sp.realtime ? 1u : 2u;
     // The cache written this tick is read by the next one.
     std::swap(d.sv_code, d.out_code);
     std::swap(d.sv_off, d.out_off);
@@ -1215,7 +1217,7 @@ int pmb_world_tick_telemetry(pmb_world* w, pmb_tick_telemetry* out) {
         out->workgroups[p] = w->ledger.workgroups[p];
     }
     const uint64_t n = w->d.n, con = c.n_contacts;
-    const uint64_t sweeps = uint64_t(c.iterations) + (c.impact ? uint64_t(c.budget) : 0u);
+    const uint64_t sweeps = uint64_t(c.iterations) + (c.impact && w->solve_phases > 1 ? uint64_t(c.budget) : 0u);
     out->sweeps = sweeps;
     out->spatial_builds = 1;
     // One barrier a colour round; in a sweep one a colour and one after the

@@ -202,19 +202,21 @@ def _telemetry(w):
     return t
 
 
+@pytest.mark.parametrize("profile", [scenes.LEGACY, scenes.REALTIME])
 @pytest.mark.parametrize("variant", [0, 3])
 @pytest.mark.parametrize("boxes", [20, 2000])
-def test_telemetry_counts_the_barriers_a_tick_passes(gpu_available, boxes, variant):
+def test_telemetry_counts_the_barriers_a_tick_passes(gpu_available, boxes, variant, profile):
     """One barrier a colour round; in a sweep one a colour and, in the group
-    variants, one after the duals. A legacy tick with an impact sweeps twice."""
+    variants, one after the duals. A legacy tick with an impact sweeps twice,
+    a realtime tick once."""
     w = core.World(scenes.box_pile((13, 13, 13), seed=5, spacing=1.4, count=boxes))
     w.set_launch_plan(variant, 0)
     for _ in range(4):
-        w.step(stats=False)
-    report = w.profile_step()
+        w.step(profile=profile, stats=False)
+    report = w.profile_step(profile=profile)
     st, t = w.stats(), _telemetry(w)
     rounds = int(re.search(r"rounds (\d+)", report).group(1))
-    sweeps = int(st["iterations"]) * (2 if st["impact"] else 1)
+    sweeps = int(st["iterations"]) * (2 if st["impact"] and profile == scenes.LEGACY else 1)
     assert rounds >= 1 and st["colors"] > 1 and t.sweeps == sweeps > 0
     assert t.barriers[4] == rounds + sweeps * (int(st["colors"]) + (1 if variant < 3 else 0))
     assert sum(t.barriers) == t.barriers[4]
