@@ -2,8 +2,8 @@
 """The tick's size-dependent branches at their edges, against the oracle.
 
 A tick picks kernels and grids by the world's size: one solve block up to 40
-bodies, narrowphase lanes up to 6,144, one-block grid and colour order up to
-8,192; a query keeps 64 candidates; a lane group takes two, five or ten joints
+bodies, narrowphase lanes up to 6,144, a one-block grid up to 8,192 buckets
+(4,096 bodies), a one-block colour order up to 8,192 bodies; a query keeps 64 candidates; a lane group takes two, five or ten joints
 of a body at a time. Every branch evaluates the serial order's operations, so states,
 candidate pairs and colours are compared bit for bit.
 """
@@ -37,7 +37,7 @@ def _same(scene, ticks, contact_capacity=0, **kw):
 
 
 # box_pile adds five static bodies; boxes 1.4 m apart touch from the start.
-@pytest.mark.parametrize("bodies", [6, 40, 41, 130, 1030, 6144, 6145, 8192, 8193])
+@pytest.mark.parametrize("bodies", [6, 40, 41, 130, 1030, 4096, 4097, 6144, 6145, 8192, 8193])
 def test_world_sizes_around_the_dispatch_edges(gpu_available, bodies):
     side = max(1, int(np.ceil((bodies - 5) ** (1.0 / 3.0))))
     scene = scenes.box_pile((side, side, side), seed=bodies, spacing=1.4, count=bodies - 5)
@@ -57,6 +57,87 @@ def test_query_with_more_candidates_than_are_kept(gpu_available):
         x, z = (k % 12 - 5.5) * 0.6, (k // 12 - 5.5) * 0.6
         b.body(cube, scenes.DYNAMIC, (x, 0.2505, z), mass=1.0, inertia=scenes.box_inertia(1.0, (0.25,) * 3))
     assert _same(b.build("plate", 10), 4) > 0
+
+
+def _plate_scene():
+    """A plate over 12 x 12 boxes, and the boxes on the ground: one query of
+    145 candidates and 144 of a few."""
+    b = scenes._Builder()
+    scenes._ground(b, 20.0, 20.0)
+    cube = b.mesh(*scenes.box_mesh((0.25, 0.25, 0.25)))
+    plate = b.mesh(*scenes.box_mesh((4.0, 0.1, 4.0)))
+    for k in range(144):
+        x, z = (k % 12 - 5.5) * 0.55, (k // 12 - 5.5) * 0.55
+        b.body(cube, scenes.DYNAMIC, (x, 0.2505, z), mass=1.0, inertia=scenes.box_inertia(1.0, (0.25,) * 3))
+        if k == 71:
+            b.body(plate, scenes.DYNAMIC, (0.0, 0.62, 0.0), mass=5.0, inertia=scenes.box_inertia(5.0, (4.0, 0.1, 4.0)))
+    return b.build("plate between", 10)
+
+
+@pytest.mark.parametrize("past", [1, 70])
+def test_a_query_cut_off_by_the_candidate_capacity(gpu_available, past):
+    """The capacity ends inside a body's segment (`past` candidates into it; 70
+    are past the kept ones): the tick reports the overflow, keeps as many
+    candidates as fit, in order and out of the full set, and goes on."""
+    scene = _plate_scene()
+    o = O.OracleWorld(scene)
+    o.step()
+    full = o.candidate_pairs()
+    query = full // scene.n
+    first, many = np.unique(query, return_index=True)[1], np.unique(query, return_counts=True)[1]
+    at = int(np.nonzero(many > past + 1)[0][-1])
+    capacity = int(first[at]) + past
+    assert many[at] > past and capacity < len(full)
+    w = core.World(scene, candidate_capacity=capacity)
+    for t in range(3):
+        st = w.step()
+        assert int(st["status"]) & 1, core.status_names(int(st["status"]))
+        assert st["candidate_pairs"] == capacity
+        codes = w.candidate_pairs()
+        assert len(codes) == capacity and (codes // scene.n < scene.n).all()
+        assert (np.diff(codes.astype(np.int64)) > 0).all()  # by query body, then by identity
+        if t == 0:
+            assert np.array_equal(codes[:first[at]], full[:first[at]])  # the whole segments before it
+            assert np.isin(codes[first[at]:], full[first[at]:first[at] + many[at]]).all()
+        assert np.isfinite(w.states()["x"]).all()
+    w.close()
+
+
+def _cone(sides, radius, height):
+    """A cone of `sides` faces, its base (y = 0) triangulated as a fan."""
+    a = 2.0 * np.pi * np.arange(sides) / sides
+    v = np.stack([radius * np.cos(a), np.zeros(sides), radius * np.sin(a)], -1)
+    v = np.concatenate([v, [[0.0, height, 0.0]]]).astype(np.float32)
+    t = [(k, (k + 1) % sides, sides) for k in range(sides)] + [(0, k, k + 1) for k in range(1, sides - 1)]
+    return v, scenes._fix_winding(v, np.array(t, np.uint32))
+
+
+@pytest.mark.parametrize("speed", [0.0, 9.0])
+def test_polygons_that_outgrow_the_lanes(gpu_available, speed):
+    """Cones of 32 triangles, the face path's most: a 17-sided base within one
+    triangle of a plate's top clips that triangle to 17 vertices, one more than
+    a pair's lanes hold. The plates come first, so at equal separations the
+    cone's base is the reference face. Resting, and falling past the margin
+    without turning (a swept pair)."""
+    sides = 17
+    v, t = _cone(sides, 1.0, 1.5)
+    assert len(t) == 96
+    b = scenes._Builder()
+    scenes._ground(b, 100.0, 100.0)
+    plate = b.mesh(*scenes.box_mesh((4.0, 0.25, 4.0)))
+    cone = b.mesh(v, t)
+    spots = [(12.0 * (k % 4), 12.0 * (k // 4)) for k in range(16)]
+    for x, z in spots:
+        b.body(plate, scenes.DYNAMIC, (x, 0.25, z), mass=200.0, inertia=scenes.box_inertia(200.0, (4.0, 0.25, 4.0)))
+    rng = np.random.Generator(np.random.Philox(5))
+    for k, (x, z) in enumerate(spots):
+        turn = float(rng.uniform(-3, 3))
+        side = 2.0 if k % 2 else -2.0  # either triangle of the plate's top
+        b.body(cone, scenes.DYNAMIC, (x + side, 0.5 + 0.09 * (speed > 0), z + side),
+               q=(0.0, float(np.sin(turn / 2)), 0.0, float(np.cos(turn / 2))), v=(0.0, -speed, 0.0), mass=2.0,
+               inertia=(0.5, 0.5, 0.5))
+    scene = b.build("cones", 10)
+    assert _same(scene, 6, contact_capacity=1 << 18) > 0
 
 
 @pytest.mark.parametrize("joints", [1, 2, 3, 5, 6, 11, 23])
