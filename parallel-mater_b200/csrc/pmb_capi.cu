@@ -174,17 +174,29 @@ __global__ void k_reset_counters(Dev d) {
 
 // The CTA size a world starts with (pmb_world_autotune measures its own).
 // Fewer threads leave each more registers (no spills, more of a chain in
-// flight) where a colour does not fill the grid anyway: 256 threads up to
-// 3,072 bodies, and up to 16,384 with joints, whose rows take the most
-// registers (us a tick with 512, 384, 256 threads: 56 bodies 457, 446, 430;
-// joint rigs, 224: 763, 729, 710; 2,202 boxes 1,180, 1,174, 1,137; 128 chains,
-// 8,448: 3,032, 2,926, 2,806). Beyond, 512 fill it (4,101 boxes 1,468, 1,498,
-// 1,473; 512 chains, 33,792: 4,584, 4,939, 5,350), but for the largest joint-
-// free worlds, many rounds a colour, 384 (65,541 boxes to a residual 24.1,
-// 23.6, 24.9 ms; 8 sweeps 5,020, 5,027, 5,195).
-uint32_t starting_variant(uint32_t bodies, uint32_t joints) {
-    if (bodies <= (joints ? 16384u : 3072u)) return 2;
-    return !joints && bodies > 32768u ? 1 : 0;
+// flight), more take more bodies at once. us a tick with 512, 384, 256 threads:
+//
+// Without joints 256 up to 3,072 bodies (56 bodies 457, 446, 430; 2,202 boxes
+// 1,180, 1,174, 1,137; 2,749: 1,239, 1,215, 1,219), then 512 (4,101: 1,139,
+// 1,135, 1,142; 8,005: 2,218, 2,249, 2,313; 30,725: 3,452, 3,533, 3,797;
+// 36,869: 3,778, 4,066, 4,221; 41,477: 4,245, 4,404, 4,576). Beyond 49,152 the
+// first two are within 4 % of each other either way (51,205: 5,156, 5,127,
+// 5,421; 81,925: 6,534, 6,776, 7,379); 384 for the denser, long-settled piles
+// (the 65,541-body benchmark pile to a residual: 21.5, 20.8, 23.7 ms).
+//
+// With joints a sweep's colours are as large as half the dynamic bodies (every
+// other link of a chain): the fewest threads whose 8-lane groups take so many
+// in one round -- 256 up to 9,472 dynamic bodies of 148 SMs (joint rigs, 144:
+// 763, 729, 710; 128 chains, 8,320: 2,478, 2,338, 2,267; 144: 2,546, 2,401,
+// 2,333), 384 up to 14,208 (160 chains, 10,400: 2,680, 2,534, 2,980; 216,
+// 14,040: 2,653, 2,506, 3,018), then 512 (232, 15,080: 2,815, 3,104, 3,163;
+// 512 chains, 33,280: 4,584, 4,939, 5,350).
+uint32_t starting_variant(const pmb_world* w, uint32_t dynamic_bodies) {
+    const uint32_t n = w->d.n;
+    if (w->d.nj == 0) return n <= 3072u ? 2 : n > 49152u ? 1 : 0;
+    for (uint32_t v = 2; v > 0; --v)
+        if (dynamic_bodies <= 2u * uint32_t(w->coop_solve[v]) * uint32_t(solve_variant(v).threads) / 8u) return v;
+    return 0;
 }
 
 // Blocks of the cooperative kernels. Few bodies need few blocks: a barrier
@@ -738,7 +750,6 @@ int pmb_world_create(const pmb_world_desc* desc, pmb_world** out) {
     std::vector<float> sorted = expand;
     std::nth_element(sorted.begin(), sorted.begin() + n / 2, sorted.end());
     d.large_extent = 2.0f * sorted[n / 2] * 4.0f;
-    d.solve_variant = starting_variant(n, nj);
     d.solve_policy = 0;
     d.barrier_spins = kDefaultBarrierSpins;
     for (uint32_t v = 0; v < kSolveVariants; ++v) {
@@ -753,6 +764,7 @@ int pmb_world_create(const pmb_world_desc* desc, pmb_world** out) {
             }
         w->coop_solve[v] = blocks;
     }
+    d.solve_variant = starting_variant(w, uint32_t(std::count(motion.begin(), motion.end(), uint32_t(kDynamic))));
     {
         int dev = 0, sms = 0;
         cudaGetDevice(&dev);
