@@ -203,11 +203,14 @@ PMB_API int pmb_world_solve_timer(pmb_world* world, int enable, float* total_ms,
  * returns PMB_ERROR_INVALID_ARGUMENT before any other device work. Work runs on `stream` (CUDA
  * stream, null for the default); the call takes scratch (104 bytes a triangle
  * and some) from a pool of the current device that keeps at most 64 MiB
- * between calls, emptied when a world of that device is destroyed, and
- * returns after the stream has finished. */
+ * between calls, emptied when a world of that device is destroyed or by
+ * pmb_mesh_bvh_release, and returns after the stream has finished. */
 PMB_API int pmb_mesh_bvh_build(const float* vertices, uint32_t vertex_count, const uint32_t* indices,
                                uint32_t index_count, uint32_t* order, float* nodes, uint32_t node_capacity,
                                uint32_t* node_count, void* stream);
+/* Gives back the scratch that the builds on `device` keep between calls; from
+ * any thread, also while others build (what they use stays theirs). */
+PMB_API int pmb_mesh_bvh_release(int32_t device);
 
 /* Host mesh preparation used at world creation (no device work): triangles
  * reordered into median-split BVH leaf order, one outward plane (n, d) per

@@ -446,8 +446,9 @@ namespace {
 // Scratch of the builds, one pool per device: cudaMalloc and cudaFree took
 // 650 us of a 1,310 us call for 200,000 triangles. The pool keeps at most
 // kPoolKept bytes between calls (more is given back when a call's stream
-// synchronises) and is emptied when a world of its device is destroyed; its
-// allocations are ordered on the caller's stream, from any thread.
+// synchronises) and is emptied when a world of its device is destroyed or by
+// pmb_mesh_bvh_release; its allocations are ordered on the caller's stream,
+// from any thread.
 constexpr uint64_t kPoolKept = uint64_t(64) << 20;
 constexpr int kPoolDevices = 64;
 std::mutex g_pool_lock;
@@ -478,6 +479,12 @@ void release_bvh_scratch(int device) {
     if (g_pools[device]) cudaMemPoolTrimTo(g_pools[device], 0);
 }
 }  // namespace pmb
+
+extern "C" int pmb_mesh_bvh_release(int32_t device) {
+    if (device < 0 || device >= kPoolDevices) return PMB_ERROR_INVALID_ARGUMENT;
+    release_bvh_scratch(device);
+    return PMB_SUCCESS;
+}
 
 extern "C" int pmb_mesh_bvh_build(const float* vertices, uint32_t vertex_count, const uint32_t* indices,
                                   uint32_t index_count, uint32_t* order, float* nodes, uint32_t node_capacity,

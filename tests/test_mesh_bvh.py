@@ -132,3 +132,43 @@ def test_device_builder_rejects_out_of_range_indices(gpu_available):
                                        d_nodes.data_ptr(), 16, ctypes.byref(count),
                                        torch.cuda.current_stream().cuda_stream)
     assert rc == -1
+
+
+def test_scratch_release_checks_its_device():
+    f = core.lib().pmb_mesh_bvh_release
+    assert f(ctypes.c_int32(-1)) == -1 and f(ctypes.c_int32(1 << 20)) == -1
+    assert f(ctypes.c_int32(0)) == 0  # nothing kept: nothing to do
+
+
+@pytest.mark.gpu
+def test_scratch_kept_between_builds_is_bounded_and_given_back(gpu_available):
+    """104 bytes of scratch a triangle: up to 64 MiB stay with the library
+    between calls, and pmb_mesh_bvh_release returns them to the device."""
+    import torch
+    release = core.lib().pmb_mesh_bvh_release
+    free = lambda: torch.cuda.mem_get_info(0)[0]
+    for triangles in (200_000, 900_000):
+        v, i = _grid_soup(triangles, 3, cells=200)
+        d_v = torch.from_numpy(v.reshape(-1)).cuda()
+        d_i = torch.from_numpy(i.view(np.int32)).cuda()
+        d_order = torch.zeros(triangles, dtype=torch.int32, device="cuda")
+        d_nodes = torch.zeros(20 * triangles, dtype=torch.int32, device="cuda")
+        count = ctypes.c_uint32()
+
+        def build():
+            rc = core.lib().pmb_mesh_bvh_build(d_v.data_ptr(), len(v), d_i.data_ptr(), len(i), d_order.data_ptr(),
+                                               d_nodes.data_ptr(), 2 * triangles, ctypes.byref(count),
+                                               torch.cuda.current_stream().cuda_stream)
+            assert rc == 0
+            return d_order.clone()
+
+        torch.cuda.synchronize()
+        build()  # (the kernels' own first-use memory)
+        assert release(ctypes.c_int32(0)) == 0
+        before = free()
+        first = build()
+        kept = before - free()
+        assert 0 < kept <= 64 << 20, kept
+        assert release(ctypes.c_int32(0)) == 0 and free() >= before
+        assert torch.equal(build(), first)
+        release(ctypes.c_int32(0))
