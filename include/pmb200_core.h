@@ -440,7 +440,9 @@ PMB_API int pmb_world_set_launch_plan(pmb_world* world, uint32_t solve_variant, 
  * kernels of the tick return at once and the host reads the status after the
  * tick (the pm* driver reports it as PM_ERROR_DEVICE_LOST); the next tick
  * starts with clean counters. A small limit makes the waits run out on
- * purpose, which is how failure detection is exercised without a GPU fault.
+ * purpose, which is how failure detection is exercised without a GPU fault: one
+ * below 1,024 polls also launches these kernels with every block the device
+ * holds at once, where a small world takes fewer (and one block has no waits).
  * Takes effect for ticks enqueued afterwards (not for graphs already
  * captured). */
 PMB_API int pmb_world_set_barrier_limit(pmb_world* world, uint32_t spins);

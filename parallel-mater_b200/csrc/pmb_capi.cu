@@ -207,17 +207,18 @@ uint32_t starting_variant(const pmb_world* w, uint32_t dynamic_bodies) {
 // threads): 22 bodies 215 with 1, 260 with 4, 334 with 148; 56 bodies 336,
 // 287, 355; 211 bodies 908 with 1, 304 with 16, 362 with 148; 1,006 bodies
 // 802 with 64, 862 with 148; 4,101 bodies 1,003 with 64, 950 with 148.
-// A world with a barrier limit of its own keeps every block, so that the
-// limit has barriers to apply to.
+// A barrier limit below kRunOutSpins polls (under a millisecond) is meant to
+// run out: every block is launched, so that a small world has barriers for it.
 constexpr uint32_t kOneBlockBodies = 40;
+constexpr uint32_t kRunOutSpins = 1024;
 int color_blocks(const pmb_world* w) {
-    if (w->d.barrier_spins != kDefaultBarrierSpins) return w->coop_color;
+    if (w->d.barrier_spins < kRunOutSpins) return w->coop_color;
     return std::min(w->coop_color, int(blocks_for(w->d.n, kColorThreads)));
 }
 int solve_blocks(const pmb_world* w) {
     const uint32_t v = w->d.solve_variant < kSolveVariants ? w->d.solve_variant : 0u;
     const int all = w->coop_solve[v];
-    if (w->d.barrier_spins != kDefaultBarrierSpins) return all;
+    if (w->d.barrier_spins < kRunOutSpins) return all;
     if (w->d.n <= kOneBlockBodies) return 1;
     const uint64_t threads = uint64_t(solve_variant(v).threads);
     return int(std::min<uint64_t>(uint64_t(all), (uint64_t(w->d.n) * 32u + threads - 1u) / threads));

@@ -299,7 +299,8 @@ class World:
 
     def set_barrier_limit(self, spins=0):
         """Polls a block makes at a grid barrier before the tick is abandoned
-        with PMB_STATUS_BARRIER_TIMEOUT (0: the default)."""
+        with PMB_STATUS_BARRIER_TIMEOUT (0: the default; below 1,024 every
+        block the device holds is launched, to have waits that run out)."""
         _check(lib().pmb_world_set_barrier_limit(self.h, spins), "set_barrier_limit")
 
     def autotune(self, desc=None, ticks=3, **kw):

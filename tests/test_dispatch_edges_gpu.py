@@ -302,3 +302,24 @@ def test_telemetry_counts_the_barriers_a_tick_passes(gpu_available, boxes, varia
     assert t.barriers[4] == rounds + sweeps * (int(st["colors"]) + (1 if variant < 3 else 0))
     assert sum(t.barriers) == t.barriers[4]
     w.close()
+
+
+@pytest.mark.parametrize("boxes", [20, 300])
+def test_a_barrier_limit_keeps_the_worlds_grid(gpu_available, boxes):
+    """A limit that can only run out by a fault leaves the launches and the
+    states as they are; one below 1,024 polls takes every block."""
+    scene = scenes.box_pile((7, 7, 7), seed=6, spacing=1.4, count=boxes)
+    states, groups = [], []
+    for limit in (0, 1 << 20):
+        w = core.World(scene)
+        w.set_barrier_limit(limit)
+        for _ in range(3):
+            assert w.step()["status"] == 0
+        states.append(w.states().view(np.uint8))
+        groups.append(list(_telemetry(w).workgroups))
+        if limit:
+            w.set_barrier_limit(1)
+            w.step()
+            assert _telemetry(w).workgroups[4] > groups[0][4] + 148
+        w.close()
+    assert np.array_equal(states[0], states[1]) and groups[0] == groups[1]
