@@ -356,7 +356,9 @@ PMB_API int pmb_world_contact_duals(pmb_world* world, uint32_t rows, float* lamb
  * contact point c (in contact order) starts from (lambda[rows*c+x],
  * penalty[rows*c+x]) for c < count and x < rows. A penalty <= 0 keeps the
  * plain penalty; a negative normal lambda or a NaN friction lambda keeps the
- * plain lambda. Copied to the device (synchronous). */
+ * plain lambda. Copied to the device (synchronous), into scratch memory: the
+ * owner of a world's scratch who writes it between ticks sets the table
+ * again. */
 PMB_API int pmb_world_set_warm_table(pmb_world* world, uint32_t rows, const float* lambda, const float* penalty,
                                      uint32_t count);
 

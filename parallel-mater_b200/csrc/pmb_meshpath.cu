@@ -683,7 +683,7 @@ __device__ __forceinline__ MeshPose pose_pred(const Dev& d, uint32_t i) {
 //   3. walk (write): the same traversal records each leaf pair and where its
 //      items start;
 //   4. items: one thread per triangle pair evaluates its contact;
-//   5. merge: one thread per pair merges its items' contacts in item order,
+//   5. merge: a warp per pair merges its items' contacts in item order,
 //      which is the reference's order, and stages them.
 constexpr uint32_t kPairSwept = 1u, kPairInteriorA = 2u, kPairInteriorB = 4u;
 

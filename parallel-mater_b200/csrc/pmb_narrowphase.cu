@@ -725,13 +725,18 @@ __device__ __forceinline__ void narrow_serial(const Dev& d, uint32_t k, uint2 sa
 __device__ __noinline__ void narrow_outgrown(const Dev& d, uint32_t k, uint2 sat) { narrow_serial(d, k, sat); }
 
 // Pass 2, a thread or 16 lanes per surviving candidate. With few survivors
-// the serial chain is what counts (217: 43 us with lanes, 124 with threads);
-// with many, the lanes' extra work (412,000: 2.36 and 0.97 ms). The survivors'
-// number is not known at the launch; piles have about six a body, so worlds of
-// up to kLaneBodies bodies take the lanes (4,096 boxes, 25,000 survivors: a
-// tick of 1,540 us against 1,658). The threads' polygons in shared memory
-// instead of local memory were slower (1.91 ms against 0.97 at 412,000): a
-// third fewer threads fit, and a warp waits for its longest polygon either way.
+// the serial chain is what counts, with many the lanes' extra work. us with
+// lanes and with threads, box piles: 126 survivors 31, 132; 4,849: 37, 175;
+// 18,302: 72, 190; 25,129 (most of them touching) 152, 219; 36,083 (likewise)
+// 226, 223; 53,710: 195, 211; 82,224: 300, 237; 412,000: 2,360, 970. The
+// survivors' number is not known at the launch; piles have four to six a body
+// (at most 37,000 in worlds of up to kLaneBodies bodies, which take the lanes).
+// Boxes spawned into one another have more: 77,731 of 2,202 bodies 294, 246.
+// (Settling it on the device cost more: a switch to threads inside the lanes'
+// kernel, whose registers leave fewer of them, 320; a kernel more, a launch in
+// every small world's tick.) The threads' polygons in shared memory instead of
+// local memory were slower (1.91 ms against 0.97 at 412,000): a third fewer
+// threads fit, and a warp waits for its longest polygon either way.
 constexpr uint32_t kLaneBodies = 6144;
 __global__ void __launch_bounds__(128, 6) k_narrow(Dev d) {
     tick_begin();

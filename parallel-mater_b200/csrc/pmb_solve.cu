@@ -827,7 +827,8 @@ __global__ void k_free_mean(Dev d, uint32_t phase) {
 }
 
 // The free islands' means taken off, then apply_states
-// (geometry_constraints_solve.slang:676-733) into the output state arrays (v: solved state; t: the AVBD target stays untouched).
+// (geometry_constraints_solve.slang:676-733) into the output state arrays
+// (v: solved state; t: the AVBD target stays untouched).
 __global__ void k_apply(Dev d, StepParams sp, uint32_t phase, float4* ox, float4* oq, float4* ov, float4* ow) {
     tick_begin();
     if (phase != 0 && d.ctr->impact == 0) return;

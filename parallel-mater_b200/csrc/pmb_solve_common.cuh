@@ -19,7 +19,8 @@ __device__ __forceinline__ Lite load_lite(const Dev& d, uint32_t i) {
 
 // Contact jacobians (geometry_constraints.slang:508-532). They depend only on
 // the contact geometry and the AVBD target poses, both fixed during a solve
-// phase, so they are evaluated once per phase and stored in the contact's phase record (d.c_row).
+// phase, so they are evaluated once per phase and stored in the contact's
+// phase record (d.c_row).
 __device__ __forceinline__ void contact_jacobians(V3 n, V3 pt, V3 anc_a, V3 anc_b, V3 xa, Q4 qa, V3 xb, Q4 qb,
                                                   V6 ja[3], V6 jb[3]) {
     V3 t0, t1;
@@ -422,9 +423,10 @@ __device__ __forceinline__ JointEnds load_ends(const Dev& d, uint32_t a, uint32_
 // the serial loop's order (joints in list order, then axes, then rows).
 // A lane takes one axis of one joint -- two, five or ten joints at a time
 // for 8, 16 and 32 lanes -- and stages its rows over the contact rows, which
-// are in the entries by now: a lane's 43 words hold three rows, the most an
-// axis of any joint but a generic or spring one has; a joint with more is
-// taken alone, its lanes' rows spread over the group's slots.
+// are in the entries by now: a lane's kSlotWords hold three rows, and only an
+// axis of a generic or spring joint, or of a piston with linear and angular
+// limits, has more; such a joint is taken alone, its lanes' rows spread over
+// the group's slots.
 constexpr int kJointWords = 12;  // jacobian[6], stiffness, force, curvature[3], whether it has one
 constexpr int kJointRowsMost = 6;
 template <int G>

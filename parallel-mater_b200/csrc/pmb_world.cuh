@@ -25,8 +25,9 @@ enum : uint32_t { kFixed, kPoint, kHinge, kSlider, kPiston, kGeneric, kGenericSp
 constexpr uint32_t kMaxColors = 256;
 constexpr uint32_t kQueryLanes = 8;  // broadphase query lanes per body
 constexpr uint32_t kQueryKept = 64;  // candidates of a body kept for the write pass
-// The colour fixpoint runs one 1024-thread CTA per SM: its ~30 rounds are
-// two grid barriers each, and a barrier's cost grows with the CTA count.
+// The colour fixpoint runs a CTA of 1,024 threads per as many bodies, at most
+// one an SM: its rounds (some 30) wait at a grid barrier each, whose cost grows
+// with the CTA count.
 constexpr int kColorThreads = 1024;
 // Sort classes of a colour's bodies by the length of their row lists,
 // heaviest first, in steps of 8 rows (an 8-lane group stages 8 rows at a
